@@ -27,9 +27,10 @@
 //
 // Scheduling: one persistent launch.  Warp w of W owns the tiles
 // w, w + W, w + 2W, ... and keeps scanning their "dirty" flags (32 at a time
-// with a ballot); a warp that relaxes a tile and changes an edge marks the
-// neighbouring tile dirty, so information crosses tile borders as soon as a
-// tile finishes, with no host round trips and no shared queue to contend on.
+// with a ballot); a warp that relaxes a tile marks a neighbouring tile dirty
+// when one of its new values would lower a pixel there, so information
+// crosses tile borders as soon as a tile finishes, with no host round trips
+// and no shared queue to contend on.
 // A tile has a single owner, so no two warps relax it at once.
 //
 // Termination: only a running warp sets flags.  A warp that finds none of
@@ -54,6 +55,13 @@ namespace {
 
 constexpr int kWarps = 4;        // tiles per block
 constexpr int kMaxSweeps = 256;  // per tile visit; a capped tile re-enqueues
+// Tiles a warp relaxes before it looks at its flags again from its lowest
+// tile on.  Few keep the warps together in one region of a large grid, whose
+// tiles are still in L2 when they are visited again; with one, a region is
+// relaxed too far on what it knows and visited more often.  16384^2, fill /
+// gwdt ms: all 32 of a poll 8.2 / 12.1, one 6.9 / 10.4, two 6.7 / 9.8, four
+// 6.9 / 9.5 (4096^2: 1.49 / 2.30, 1.45 / 2.10, 1.44 / 2.15, 1.43 / 2.14).
+constexpr int kTakeTiles = 4;
 constexpr float kSqrt2 = 1.41421356237309504880f;
 
 // GWDT_HALF: gwdt over costs stored halved (the pipeline's own costs, at
@@ -63,14 +71,21 @@ constexpr float kSqrt2 = 1.41421356237309504880f;
 enum Kind { FILL = 0, GWDT = 1, GWDT_HALF = 2 };
 
 struct WarpTile {
+  float before[kPitch];    // a sweep's last step prefetches one position past
   float s[kHalo][kPitch];  // state: f (fill) or dist (gwdt); [c][r]
   float a[kHalo][kPitch];  // aux: dem (fill) or costs (gwdt)
+  float after[kPitch];     // the halo, on either side
+  // Word offsets of s[c][r] and a[c][r] in the tile (c, r from -1 to kHalo).
+  static constexpr int s_at(int c, int r) { return (c + 1) * kPitch + r; }
+  static constexpr int a_at(int c, int r) { return (c + 1 + kHalo) * kPitch + r; }
 };
+static_assert(sizeof(WarpTile) == (2 * kHalo + 2) * kPitch * sizeof(float), "packed rows");
 
 // Control block (device memory, zero-initialised).
 struct QueueCtl {
   unsigned long long visits;  // tiles relaxed so far (flushed in batches)
   unsigned long long idle;    // wakes << 32 | warps that found nothing to do
+  // done and abort are polled with one 8-byte load
   int done;                   // set once every warp is idle and no flag is set
   int abort;                  // ABORT_* bits
   int thresh;                 // ordered schedules: tiles with priority <= thresh run
@@ -127,15 +142,29 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// Transpose of a 32 x 32 bit matrix held one row per lane.
+// Transpose of a 32 x 32 bit matrix held one row per lane: five exchanges
+// of half blocks between lanes (five shuffles instead of 32 ballots).
 __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
-  uint32_t y = 0;
+  uint32_t mask = 0x0000ffffu;
 #pragma unroll
-  for (int k = 0; k < 32; k++) {
-    const uint32_t b = __ballot_sync(0xffffffffu, (x >> k) & 1u);
-    if (lane == k) y = b;
+  for (int j = 16; j; j >>= 1, mask ^= mask << j) {
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+    x = (lane & j) ? ((x & ~mask) | ((y >> j) & mask)) : ((x & mask) | ((y & mask) << j));
   }
-  return y;
+  return x;
+}
+
+// Three-input minimum, ignoring NaN like fminf.
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// Maximum that is NaN when either operand is.
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
 }
 
 // One Gauss-Seidel sweep.  Each lane carries one line of the tile: a column
@@ -146,21 +175,39 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
 // live in registers, bit k = k-th pixel of the line.
 //
 // A step (one pixel per lane) evaluates every lane's pixel: in SIMT that
-// costs the same as evaluating only the marked ones, and it keeps the
-// per-step dependency chain down to the loads and the minimum.  After the
-// sweep a pixel is marked again if a neighbour evaluated in the same step or
-// a later one changed (neighbours of earlier steps were already final when
-// it was evaluated), and unevaluated pixels keep their marks.  An unmarked
+// costs the same as evaluating only the marked ones.  After the sweep a
+// pixel is marked again if a neighbour evaluated in the same step or a
+// later one changed (neighbours of earlier steps were already final when it
+// was evaluated), and unevaluated pixels keep their marks.  An unmarked
 // pixel therefore cannot be lowered by any neighbour, and the tile is at its
 // local fixpoint exactly when no pixel is marked.  Neighbour values may be
 // old or new: every value is an upper bound of the fixpoint, so any mix
 // gives a valid (and never higher) result.
 //
-// Both kinds run every step from the first marked one to the end of the
-// line with no vote at all: a per-step vote would put a warp-wide round trip
-// on the chain between steps.
-__device__ __forceinline__ void remark(int lane, int dir, uint32_t dm, uint32_t evald,
-                                       uint32_t &nd, uint32_t &dm_all) {
+// The sweeps took 177 cycles a step on an idle SM and 291 (fill) to 380
+// (gwdt) on a busy one with a branch around the store, a barrier and the
+// loads of the same step on the chain; in the form below they take 82 and
+// 179 to 222 (16384^2 gwdt 13.4 -> 12.2 ms, 4096^2 3.4 -> 2.4 ms).
+//
+// What bounds a sweep is the chain from one step's results to the next
+// step's inputs, on small grids and at the end of every run, and the issue
+// slots where every warp is busy.  So the chain holds only what depends on
+// the previous step: the lane's own previous result and those of the two
+// adjacent lanes (two shuffles; for the outer lanes the halo line's value,
+// which no step changes), one three-input minimum, the minimum with
+// everything else, and the centre's own update.  All other operands are
+// read from shared memory one step ahead, results are stored without being
+// read again in the same sweep (no barrier between steps), and the changed
+// bits are shifted into a mask.  Sweeps start at the group of kSweepUnroll
+// steps that holds the first marked one (evaluating an unmarked pixel
+// changes nothing).
+constexpr int kSweepUnroll = 4;
+
+__device__ __forceinline__ void remark(int lane, int first, int dir, uint32_t dm, uint32_t &nd,
+                                       uint32_t &dm_all) {
+  // steps shifted their bits in from below: the first step's bit is highest
+  if (dir > 0) dm = __brev(dm);
+  const uint32_t evald = dir > 0 ? 0xffffffffu << first : 0xffffffffu >> first;
   const uint32_t from_prev = __shfl_up_sync(0xffffffffu, dm, 1);
   const uint32_t from_next = __shfl_down_sync(0xffffffffu, dm, 1);
   const uint32_t side = (lane > 0 ? from_prev : 0u) | (lane < 31 ? from_next : 0u);
@@ -170,152 +217,177 @@ __device__ __forceinline__ void remark(int lane, int dir, uint32_t dm, uint32_t 
   dm_all |= dm;
 }
 
-// Fill sweep.  A step reads what an evaluation after the previous step's
-// stores would read, but carries part of it in registers: the lane's own
-// pixel behind (its previous result), its own pixel and the adjacent lines'
-// pixels at the current position (read one step ahead; only this step
-// writes them).  It loads only the adjacent lines' pixels behind (written by
-// the previous step) and the three pixels ahead: five state loads a step
-// instead of nine, on the shared-memory pipe that all warps of an SM share.
-template <bool ALONG_C>
-__device__ __forceinline__ void sweep_fill(WarpTile &t, int lane, int dir, uint32_t &nd,
-                                           uint32_t &dm_all) {
+// First step of a sweep over the marks `nd` (32: nothing marked).
+__device__ __forceinline__ int first_step(uint32_t nd, int dir) {
   const uint32_t steps = __reduce_or_sync(0xffffffffu, nd);
-  if (!steps) return;
-  const int first = dir > 0 ? __ffs(steps) - 1 : kTile - 1 - (31 - __clz(steps));
+  if (!steps) return kTile;
+  return (dir > 0 ? __ffs(steps) - 1 : __clz(steps)) & ~(kSweepUnroll - 1);
+}
+
+// chamfer * (c(u) + c(v)) / 2 between side and corner neighbours;
+// multiplying by 1 is exact (HALF: the costs are already halved).
+template <bool HALF>
+__device__ __forceinline__ float side_weight(float c, float d) {
+  return HALF ? __fadd_rn(c, d) : __fmul_rn(__fadd_rn(c, d), 0.5f);
+}
+template <bool HALF>
+__device__ __forceinline__ float diag_weight(float c, float d) {
+  return HALF ? __fmul_rn(kSqrt2, __fadd_rn(c, d))
+              : __fmul_rn(__fmul_rn(kSqrt2, __fadd_rn(c, d)), 0.5f);
+}
+
+// Fill sweep: f = max(z, min of the 3 x 3 neighbourhood).  A NaN pixel is
+// NaN in state and elevation: it is ignored by its neighbours' minima and
+// stays NaN.
+template <bool ALONG_C, int DIR>
+__device__ __forceinline__ void sweep_fill(WarpTile &t, int lane, uint32_t &nd,
+                                           uint32_t &dm_all) {
+  const int first = first_step(nd, DIR);
+  if (first >= kTile) return;
   // Pixel (line l, position p): t.s[l][p] in the column layout, t.s[p][l]
   // in the row layout.  The lane's line is l = lane + 1.
   constexpr int PS = ALONG_C ? kPitch : 1;  // between positions
   constexpr int LS = ALONG_C ? 1 : kPitch;  // between lines
-  float *const sline = ALONG_C ? &t.s[0][lane + 1] : &t.s[lane + 1][0];
-  const float *const aline = ALONG_C ? &t.a[0][lane + 1] : &t.a[lane + 1][0];
-  const int D = dir * PS;  // to the next position of the sweep
-  uint32_t dm = 0, evald = 0;
-  float ob = 0.f, op = 0.f, lp = 0.f, rp = 0.f;  // own behind / here, adjacent here
-  bool have = false;  // the registers hold the previous step's values
+  constexpr int D = DIR * PS;               // to the next position of the sweep
+  const int p0 = (DIR > 0 ? first : kTile - 1 - first) + 1;
+  float *sp = reinterpret_cast<float *>(&t) +
+              (ALONG_C ? WarpTile::s_at(p0, lane + 1) : WarpTile::s_at(lane + 1, p0));
+  const float *ap = reinterpret_cast<const float *>(&t) +
+                    (ALONG_C ? WarpTile::a_at(p0, lane + 1) : WarpTile::a_at(lane + 1, p0));
+  uint32_t dm = 0;
+  const bool lo_lane = lane == 0, hi_lane = lane == kTile - 1;
+  float lh = sp[-LS - D], rh = sp[LS - D];  // adjacent lines behind (the halo's for the outer lanes)
+  float ob = sp[-D];                        // own pixel behind
+  float lp = sp[-LS], op = sp[0], rp = sp[LS], z = ap[0];  // here
+  float la = sp[-LS + D], oa = sp[D], ra = sp[LS + D];     // ahead
 #pragma unroll 1
-  for (int s = first; s < kTile; s++) {
-    const int k = dir > 0 ? s : kTile - 1 - s;  // position along the line
-    const uint32_t bit = 1u << k;
-    evald |= bit;
-    float *const sp = sline + (k + 1) * PS;
-    if (!have) {
-      ob = sp[-D];
-      op = sp[0];
-      lp = sp[-LS];
-      rp = sp[LS];
+  for (int s = first; s < kTile; s += kSweepUnroll) {
+#pragma unroll
+    for (int u = 0; u < kSweepUnroll; u++) {
+      // the next step's row ahead and centre (the last step reads past the
+      // halo, inside the tile arrays, and its values are not used)
+      const float la2 = sp[-LS + 2 * D], oa2 = sp[2 * D], ra2 = sp[LS + 2 * D], z2 = ap[D];
+      const float ls = __shfl_up_sync(0xffffffffu, ob, 1);
+      const float rs = __shfl_down_sync(0xffffffffu, ob, 1);
+      const float pre = min3(min3(op, lp, rp), min3(la, oa, ra), ob);
+      const float nv = max_nan(z, min3(pre, lo_lane ? lh : ls, hi_lane ? rh : rs));
+      const bool ch = nv < op;
+      if (ch) sp[0] = nv;
+      dm = dm + dm + (ch ? 1u : 0u);
+      ob = nv;  // nv == op where it is not lower (f >= z throughout)
+      lh = lp;
+      rh = rp;
+      lp = la;
+      op = oa;
+      rp = ra;
+      la = la2;
+      oa = oa2;
+      ra = ra2;
+      z = z2;
+      sp += D;
+      ap += D;
     }
-    const float lb = sp[-LS - D], rb = sp[LS - D];  // written by the previous step
-    const float oa = sp[D], la = sp[-LS + D], ra = sp[LS + D];
-    const float cur = op;
-    const float z = aline[(k + 1) * PS];
-    const float a0 = fminf(lb, lp), a1 = fminf(la, ob);
-    const float a2 = fminf(oa, rb), a3 = fminf(rp, ra);
-    const float lo = fminf(cur, fminf(fminf(a0, a1), fminf(a2, a3)));
-    const float nv = (lo > z) ? lo : z;
-    const bool ch = nv < cur;
-    if (ch) {
-      sp[0] = nv;
-      dm |= bit;
-    }
-    ob = ch ? nv : cur;
-    op = oa;
-    lp = la;
-    rp = ra;
-    have = true;
-    __syncwarp();
   }
-  remark(lane, dir, dm, evald, nd, dm_all);
+  __syncwarp();  // the stores before the next sweep's loads
+  remark(lane, first, DIR, dm, nd, dm_all);
 }
 
-// Gwdt sweep in the fill's form: every step from the first marked one to
-// the end of the line, no votes, with the values a step would re-read
-// unchanged carried in registers (state of the lane's own pixel behind and
-// here, adjacent lines here; costs of all three lines behind and here).
-// Non-flat and off-grid pixels are staged with cost NaN (state 0 or +INF):
-// every path through them evaluates to NaN, which never wins the minimum,
-// and a non-flat centre (cost NaN) keeps its value.
-template <bool ALONG_C, bool HALF>
-__device__ __forceinline__ void sweep_gwdt_run(WarpTile &t, int lane, int dir, uint32_t &nd,
-                                               uint32_t &dm_all) {
-  const uint32_t steps = __reduce_or_sync(0xffffffffu, nd);
-  if (!steps) return;
-  const int first = dir > 0 ? __ffs(steps) - 1 : kTile - 1 - (31 - __clz(steps));
+// Gwdt sweep in the fill's form, with the costs of all three lines behind,
+// here and ahead in registers.  Non-flat and off-grid pixels are staged with
+// cost NaN (state 0 or +INF): every path through them evaluates to NaN,
+// which never wins the minimum, and a non-flat centre (cost NaN) keeps its
+// value.
+template <bool ALONG_C, int DIR, bool HALF>
+__device__ __forceinline__ void sweep_gwdt(WarpTile &t, int lane, uint32_t &nd,
+                                           uint32_t &dm_all) {
+  const int first = first_step(nd, DIR);
+  if (first >= kTile) return;
   constexpr int PS = ALONG_C ? kPitch : 1;
   constexpr int LS = ALONG_C ? 1 : kPitch;
-  float *const sline = ALONG_C ? &t.s[0][lane + 1] : &t.s[lane + 1][0];
-  const float *const aline = ALONG_C ? &t.a[0][lane + 1] : &t.a[lane + 1][0];
-  const int D = dir * PS;
-  uint32_t dm = 0, evald = 0;
-  float ob = 0.f, op = 0.f, lp = 0.f, rp = 0.f;
-  float cb0 = 0.f, cb1 = 0.f, cb2 = 0.f, cp0 = 0.f, cp1 = 0.f, cp2 = 0.f;
-  bool have = false;
+  constexpr int D = DIR * PS;
+  const int p0 = (DIR > 0 ? first : kTile - 1 - first) + 1;
+  float *sp = reinterpret_cast<float *>(&t) +
+              (ALONG_C ? WarpTile::s_at(p0, lane + 1) : WarpTile::s_at(lane + 1, p0));
+  const float *ap = reinterpret_cast<const float *>(&t) +
+                    (ALONG_C ? WarpTile::a_at(p0, lane + 1) : WarpTile::a_at(lane + 1, p0));
+  uint32_t dm = 0;
+  const bool lo_lane = lane == 0, hi_lane = lane == kTile - 1;
+  auto side = [](float c, float d) { return side_weight<HALF>(c, d); };
+  auto diag = [](float c, float d) { return diag_weight<HALF>(c, d); };
+  float lh = sp[-LS - D], rh = sp[LS - D], ob = sp[-D];
+  float lp = sp[-LS], op = sp[0], rp = sp[LS];
+  float la = sp[-LS + D], oa = sp[D], ra = sp[LS + D];
+  float cb0 = ap[-LS - D], cb2 = ap[LS - D];
+  float cp0 = ap[-LS], cp1 = ap[0], cp2 = ap[LS];
+  float ca0 = ap[-LS + D], ca1 = ap[D], ca2 = ap[LS + D];
+  float wb = side(cp1, ap[-D]);  // own line: between behind and here
 #pragma unroll 1
-  for (int s = first; s < kTile; s++) {
-    const int k = dir > 0 ? s : kTile - 1 - s;
-    const uint32_t bit = 1u << k;
-    evald |= bit;
-    float *const sp = sline + (k + 1) * PS;
-    const float *const ap = aline + (k + 1) * PS;
-    if (!have) {
-      ob = sp[-D];
-      op = sp[0];
-      lp = sp[-LS];
-      rp = sp[LS];
-      cb0 = ap[-LS - D];
-      cb1 = ap[-D];
-      cb2 = ap[LS - D];
-      cp0 = ap[-LS];
-      cp1 = ap[0];
-      cp2 = ap[LS];
+  for (int s = first; s < kTile; s += kSweepUnroll) {
+#pragma unroll
+    for (int u = 0; u < kSweepUnroll; u++) {
+      const float la2 = sp[-LS + 2 * D], oa2 = sp[2 * D], ra2 = sp[LS + 2 * D];
+      const float d0 = ap[-LS + 2 * D], d1 = ap[2 * D], d2 = ap[LS + 2 * D];
+      const float ls = __shfl_up_sync(0xffffffffu, ob, 1);
+      const float rs = __shfl_down_sync(0xffffffffu, ob, 1);
+      const float wa = side(cp1, ca1);
+      const float wl = diag(cp1, cb0), wr = diag(cp1, cb2);
+      float pre = min3(op, __fadd_rn(oa, wa), __fadd_rn(lp, side(cp1, cp0)));
+      pre = min3(pre, __fadd_rn(rp, side(cp1, cp2)), __fadd_rn(la, diag(cp1, ca0)));
+      pre = min3(pre, __fadd_rn(ra, diag(cp1, ca2)), __fadd_rn(ob, wb));
+      const float nv = min3(pre, __fadd_rn(lo_lane ? lh : ls, wl),
+                            __fadd_rn(hi_lane ? rh : rs, wr));
+      const bool ch = nv < op;
+      if (ch) sp[0] = nv;
+      dm = dm + dm + (ch ? 1u : 0u);
+      ob = nv;
+      lh = lp;
+      rh = rp;
+      lp = la;
+      op = oa;
+      rp = ra;
+      la = la2;
+      oa = oa2;
+      ra = ra2;
+      cb0 = cp0;
+      cb2 = cp2;
+      cp0 = ca0;
+      cp1 = ca1;
+      cp2 = ca2;
+      ca0 = d0;
+      ca1 = d1;
+      ca2 = d2;
+      wb = wa;
+      sp += D;
+      ap += D;
     }
-    const float lb = sp[-LS - D], rb = sp[LS - D];  // written by the previous step
-    const float oa = sp[D], la = sp[-LS + D], ra = sp[LS + D];
-    const float ca0 = ap[-LS + D], ca1 = ap[D], ca2 = ap[LS + D];
-    const float cur = op, cs = cp1;
-    // d(u) + chamfer * (c(u) + c(v)) / 2; multiplying by 1 is exact (HALF:
-    // the costs are already halved)
-    auto side = [&](float d, float c) {
-      return HALF ? __fadd_rn(d, __fadd_rn(cs, c))
-                  : __fadd_rn(d, __fmul_rn(__fadd_rn(cs, c), 0.5f));
-    };
-    auto diag = [&](float d, float c) {
-      return HALF ? __fadd_rn(d, __fmul_rn(kSqrt2, __fadd_rn(cs, c)))
-                  : __fadd_rn(d, __fmul_rn(__fmul_rn(kSqrt2, __fadd_rn(cs, c)), 0.5f));
-    };
-    float best = fminf(cur, fminf(side(oa, ca1), side(lp, cp0)));
-    best = fminf(best, fminf(side(rp, cp2), diag(la, ca0)));
-    best = fminf(best, diag(ra, ca2));
-    best = fminf(best, fminf(side(ob, cb1), fminf(diag(lb, cb0), diag(rb, cb2))));
-    const float nv = best;
-    const bool ch = nv < cur;
-    if (ch) {
-      sp[0] = nv;
-      dm |= bit;
-    }
-    ob = ch ? nv : cur;
-    op = oa;
-    lp = la;
-    rp = ra;
-    cb0 = cp0;
-    cb1 = cp1;
-    cb2 = cp2;
-    cp0 = ca0;
-    cp1 = ca1;
-    cp2 = ca2;
-    have = true;
-    __syncwarp();
   }
-  remark(lane, dir, dm, evald, nd, dm_all);
+  __syncwarp();
+  remark(lane, first, DIR, dm, nd, dm_all);
 }
 
-template <int KIND, bool ALONG_C>
-__device__ __forceinline__ void sweep(WarpTile &t, int lane, int dir, uint32_t &nd,
-                                      uint32_t &dm_all) {
+template <int KIND, bool ALONG_C, int DIR>
+__device__ __forceinline__ void sweep(WarpTile &t, int lane, uint32_t &nd, uint32_t &dm_all) {
   if (KIND == FILL)
-    sweep_fill<ALONG_C>(t, lane, dir, nd, dm_all);
+    sweep_fill<ALONG_C, DIR>(t, lane, nd, dm_all);
   else
-    sweep_gwdt_run<ALONG_C, KIND == GWDT_HALF>(t, lane, dir, nd, dm_all);
+    sweep_gwdt<ALONG_C, DIR, KIND == GWDT_HALF>(t, lane, nd, dm_all);
+}
+
+// Whether the tile's values would lower the halo pixel at word `q` of the
+// tile: `n` is the pixel of the tile beside it, `along` the stride along the
+// edge (the three pixels n - along, n, n + along touch q), 0 for a corner of
+// the halo (n alone touches it).
+template <int KIND>
+__device__ __forceinline__ bool lowers(const WarpTile &t, int q, int n, int along) {
+  const float *const s = reinterpret_cast<const float *>(&t);
+  const float *const a = s + kHalo * kPitch;
+  constexpr bool HALF = KIND == GWDT_HALF;
+  if (KIND == FILL)
+    return max_nan(a[q], along ? min3(s[n - along], s[n], s[n + along]) : s[n]) < s[q];
+  if (!along) return __fadd_rn(s[n], diag_weight<HALF>(a[q], a[n])) < s[q];
+  return min3(__fadd_rn(s[n - along], diag_weight<HALF>(a[q], a[n - along])),
+              __fadd_rn(s[n], side_weight<HALF>(a[q], a[n])),
+              __fadd_rn(s[n + along], diag_weight<HALF>(a[q], a[n + along]))) < s[q];
 }
 
 // Sweep schedules (a template parameter, picked at run time): bit 0 runs the
@@ -384,21 +456,25 @@ relax_persistent_kernel(RelaxArgs a) {
   int posted = kClean;               // ordered: this warp's last wmin entry
   int raised_at = kUrgent;           // ordered: threshold this warp last raised from
   for (;;) {
-    if (*(volatile int *)&a.ctl->abort || *(volatile int *)&a.ctl->done) break;
+    // The stop word and the first flags are loaded together: a poll costs
+    // one round trip to L2, which is on the path of every change that
+    // crosses tiles.
+    const unsigned long long stop_word = *(volatile unsigned long long *)&a.ctl->done;
+    int f0 = wid + lane * W < T ? *(volatile int *)&a.dirty[wid + lane * W] : 0;
     const int thr = ordered_sched(SCHED) ? *(volatile int *)&a.ctl->thresh : 0;
+    if (stop_word) break;
     int lane_wait = kClean;  // ordered: lowest priority of this lane's waiting tiles
-    if (lane == 0) {
-      if (unflushed >= (unsigned long long)a.visit_flush) {
-        atomicAdd(&a.ctl->visits, unflushed);
-        unflushed = 0;
-      }
-      if (*(volatile unsigned long long *)&a.ctl->visits >= a.max_visits)
+    if (lane == 0 && unflushed >= (unsigned long long)a.visit_flush) {
+      if (atomicAdd(&a.ctl->visits, unflushed) + unflushed >= a.max_visits)
         atomicOr(&a.ctl->abort, ABORT_VISITS);
+      unflushed = 0;
     }
     bool did = false;
+    int taken = 0;
     for (int base = wid; base < T; base += W * 32) {
       const int mine = base + lane * W;
-      int f = (mine < T) ? *(volatile int *)&a.dirty[mine] : 0;
+      int f = f0;
+      if (base != wid) f = (mine < T) ? *(volatile int *)&a.dirty[mine] : 0;
       bool elig = f != 0;
       if (ordered_sched(SCHED) && elig) {
         const int pr = *(volatile int *)&a.prio[mine];
@@ -437,7 +513,9 @@ relax_persistent_kernel(RelaxArgs a) {
         if (!got) continue;
         did = true;
         relax_tile<KIND, SCHED>(a, t, lane, tile, got);
+        if (++taken == kTakeTiles) break;
       }
+      if (taken == kTakeTiles) break;
     }
     int wait_min = kClean;
     if (ordered_sched(SCHED)) {  // report this warp's waiting work
@@ -478,7 +556,8 @@ relax_persistent_kernel(RelaxArgs a) {
         atomicOr(&a.ctl->abort, ABORT_SPIN);
         stop = 1;
       } else {
-        __nanosleep(spins < 64 ? 64 : 512);
+        // a warp that owns one tile waits on one flag: it polls at once
+        if (T > W || spins > 256) __nanosleep(spins < 64 ? 64 : 512);
       }
     }
     if (__shfl_sync(0xffffffffu, stop, 0)) break;
@@ -510,6 +589,24 @@ __device__ void relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
   const int rx = kTile + (lane & 1);  // halo row 32 or 33
   const int64_t ix = i0 - 1 + rx;
   const bool ix_ok = ix < a.m;
+  if (i0 >= 1 && j0 >= 1 && i0 + kTile < a.m && j0 + kTile < a.n) {
+    // the tile and its halo lie on the grid (a grid has below 2^31 pixels)
+    const int m = (int)a.m, q0 = (int)((j0 - 1) * a.m + im);
+    const int qx = (int)((j0 - 1 + (lane >> 1)) * a.m + ix);
+#pragma unroll
+    for (int c = 0; c < kHalo; c++) {
+      sv[c] = __ldcg(&a.state[q0 + c * m]);
+      cp_async4(&t.a[c][lane], &a.aux[q0 + c * m]);
+    }
+#pragma unroll
+    for (int u = 0; u < 3; u++) {
+      const int c = (lane >> 1) + 16 * u;
+      if (c < kHalo) {
+        sx[u] = __ldcg(&a.state[qx + 16 * u * m]);
+        cp_async4(&t.a[c][rx], &a.aux[qx + 16 * u * m]);
+      }
+    }
+  } else {
 #pragma unroll
   for (int c = 0; c < kHalo; c++) {
     const int64_t j = j0 - 1 + c;
@@ -537,6 +634,7 @@ __device__ void relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
       }
     }
   }
+  }
 #pragma unroll
   for (int c = 0; c < kHalo; c++) t.s[c][lane] = sv[c];
 #pragma unroll
@@ -551,7 +649,7 @@ __device__ void relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
   // interior row k + 1.  An edge visit starts from the ring next to the halo.
   uint32_t nd = ((mode & DIRTY_FULL) || lane == 0 || lane == kTile - 1) ? 0xffffffffu
                                                                        : 0x80000001u;
-  uint32_t dm = 0;
+  uint32_t dm = 0, dmr = 0;  // changed pixels, column and row layout
 
   // Sweep until no pixel is marked for re-evaluation: the local fixpoint.
   // Down and up run in the column layout, right and left in the row layout
@@ -560,15 +658,14 @@ __device__ void relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
   bool done = false;
   int sweeps = 0;
   auto rows = [&]() {  // right and left in the row layout
-    uint32_t ndr = transpose32(nd, lane), dmr = 0;
-    sweep<KIND, true>(t, lane, +1, ndr, dmr);
+    uint32_t ndr = transpose32(nd, lane);
+    sweep<KIND, true, +1>(t, lane, ndr, dmr);
     sweeps++;
     if (__any_sync(0xffffffffu, ndr != 0)) {
-      sweep<KIND, true>(t, lane, -1, ndr, dmr);
+      sweep<KIND, true, -1>(t, lane, ndr, dmr);
       sweeps++;
     }
     nd = transpose32(ndr, lane);
-    dm |= transpose32(dmr, lane);
   };
   while (sweeps < kCap) {
     if (!__any_sync(0xffffffffu, nd != 0)) {
@@ -582,13 +679,13 @@ __device__ void relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
         break;
       }
     }
-    sweep<KIND, false>(t, lane, +1, nd, dm);
+    sweep<KIND, false, +1>(t, lane, nd, dm);
     sweeps++;
     if (!__any_sync(0xffffffffu, nd != 0)) {
       done = true;
       break;
     }
-    sweep<KIND, false>(t, lane, -1, nd, dm);
+    sweep<KIND, false, -1>(t, lane, nd, dm);
     sweeps++;
     if (ordered_sched(SCHED) || !(SCHED & 1)) {
       if (!__any_sync(0xffffffffu, nd != 0)) {
@@ -599,34 +696,54 @@ __device__ void relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
     }
   }
 
-  // Write back changed cells (coalesced per column: lane = row).
-#pragma unroll 4
-  for (int c = 0; c < kTile; c++) {
-    const uint32_t d = __shfl_sync(0xffffffffu, dm, c);
-    if (!d) continue;
-    if ((d >> lane) & 1u) {
-      const int64_t j = j0 + c, i = i0 + lane;
-      if (j < a.n && i < a.m) a.state[j * a.m + i] = t.s[c + 1][lane + 1];
+  // Write back changed cells, coalesced per column: lane = row, bit c of
+  // `dmr` = column c.  (Off-grid cells never change.)
+  dmr |= transpose32(dm, lane);
+  const uint32_t cols = __reduce_or_sync(0xffffffffu, dmr);
+  if (!cols && done) return;
+  {
+    float *const out = a.state + (j0 * a.m + i0 + lane);
+#pragma unroll 1
+    for (int c0 = 0; c0 < kTile; c0 += 8) {
+      if (!((cols >> c0) & 0xffu)) continue;
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        if ((dmr >> (c0 + u)) & 1u) out[(c0 + u) * a.m] = t.s[c0 + u + 1][lane + 1];
     }
   }
-  const bool top = __any_sync(0xffffffffu, dm & 1u);
-  const bool bottom = __any_sync(0xffffffffu, (dm >> 31) & 1u);
-  const uint32_t left = __shfl_sync(0xffffffffu, dm, 0);
-  const uint32_t right = __shfl_sync(0xffffffffu, dm, kTile - 1);
+  // A neighbour needs a visit only if a value of this tile lowers a pixel of
+  // it: the halo holds its values as they were staged, and they only fall,
+  // so a pixel that is not lowered here cannot be lowered there either.
+  // (Four to five in ten visits found nothing to lower without this test:
+  // 16384^2 fill 7.4 -> 6.9 ms, gwdt 11.9 -> 10.4 ms.)
+  constexpr auto at = WarpTile::s_at;
+  const uint32_t row0 = __shfl_sync(0xffffffffu, dmr, 0);
+  const uint32_t row31 = __shfl_sync(0xffffffffu, dmr, kTile - 1);
+  const uint32_t left = __ballot_sync(0xffffffffu, dmr & 1u);
+  const uint32_t right = __ballot_sync(0xffffffffu, dmr >> 31);
+  const bool to_top = row0 && __any_sync(0xffffffffu, lowers<KIND>(t, at(lane + 1, 0), at(lane + 1, 1), kPitch));
+  const bool to_bottom =
+      row31 && __any_sync(0xffffffffu, lowers<KIND>(t, at(lane + 1, kTile + 1), at(lane + 1, kTile), kPitch));
+  const bool to_left = left && __any_sync(0xffffffffu, lowers<KIND>(t, at(0, lane + 1), at(1, lane + 1), 1));
+  const bool to_right =
+      right && __any_sync(0xffffffffu, lowers<KIND>(t, at(kTile + 1, lane + 1), at(kTile, lane + 1), 1));
 
   // Lanes 0..8 mark one neighbour each with an atomic OR, after a release
   // fence.  A tile whose edges did not change publishes nothing: only its
   // owner reads its interior again.
   int tgt = -1, val = DIRTY_EDGE;
   switch (lane) {
-    case 0: if (top) { tgt = 0; } break;
-    case 1: if (bottom) { tgt = 1; } break;
-    case 2: if (left) { tgt = 2; } break;
-    case 3: if (right) { tgt = 3; } break;
-    case 4: if (left & 1u) { tgt = 4; } break;
-    case 5: if ((left >> 31) & 1u) { tgt = 5; } break;
-    case 6: if (right & 1u) { tgt = 6; } break;
-    case 7: if ((right >> 31) & 1u) { tgt = 7; } break;
+    case 0: if (to_top) { tgt = 0; } break;
+    case 1: if (to_bottom) { tgt = 1; } break;
+    case 2: if (to_left) { tgt = 2; } break;
+    case 3: if (to_right) { tgt = 3; } break;
+    case 4: case 5: case 6: case 7: {  // corners: column 0 / 31, row 0 / 31
+      const int c = lane < 6 ? 0 : kTile + 1, r = (lane & 1) ? kTile + 1 : 0;
+      const int cn = lane < 6 ? 1 : kTile, rn = (lane & 1) ? kTile : 1;
+      const uint32_t edge = lane < 6 ? left : right;
+      if (((edge >> (rn - 1)) & 1u) && lowers<KIND>(t, at(c, r), at(cn, rn), 0)) tgt = lane;
+      break;
+    }
     case 8: if (!done) { tgt = 8; val = DIRTY_FULL; } break;  // capped: revisit
     default: break;
   }
@@ -644,8 +761,8 @@ __device__ void relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
   int key = kUrgent;
   if (ordered_sched(SCHED)) {  // the lowest changed value on the tile's edges
     float v = INFINITY;
-    if (dm & 1u) v = fminf(v, t.s[lane + 1][1]);
-    if ((dm >> 31) & 1u) v = fminf(v, t.s[lane + 1][kTile]);
+    if ((row0 >> lane) & 1u) v = fminf(v, t.s[lane + 1][1]);
+    if ((row31 >> lane) & 1u) v = fminf(v, t.s[lane + 1][kTile]);
     if ((left >> lane) & 1u) v = fminf(v, t.s[1][lane + 1]);
     if ((right >> lane) & 1u) v = fminf(v, t.s[kTile][lane + 1]);
     key = __reduce_min_sync(0xffffffffu, value_key(v));
