@@ -466,8 +466,8 @@ tt_cuda_status accumulate_edgelist_dev(float *acc, const ptrdiff_t *source,
   // get a stream-ordered allocation of their own.
   uint8_t *dir = nullptr;
   int *seen = nullptr, *maxin = nullptr, *err = nullptr;
-  TT_CHECK(cudaMallocAsync((void **)&dir, (size_t)N + 256, st));
-  TT_CHECK(cudaMallocAsync((void **)&seen, (size_t)N * 8 + 256, st));
+  TT_CHECK(stream_alloc((void **)&dir, (size_t)N + 256, st));
+  TT_CHECK(stream_alloc((void **)&seen, (size_t)N * 8 + 256, st));
   maxin = seen + N;
   err = seen + 2 * N;
   TT_CHECK(cudaMemsetAsync(dir, 0, (size_t)N, st));

@@ -1040,6 +1040,7 @@ struct UpWork {
   int *xmap, *xsteps, *elist, *leaves, *h;
   long long *raw;  // passes * N fixed-point totals (multi-scale sums only)
   int *counters;  // [0] ecount, [1] lcount, [2] processed, [3] hmax, [4] err
+  bool in_arena;  // counters: a cleared status block of the pipeline call
   int *plan;      // [0..2] deferred weighted sums' {passes, k1, d}, [4..5] their range,
                   // [8] the maximum height, kept from the pass that computed it
 };
@@ -1052,8 +1053,10 @@ tt_cuda_status keep_hmax(UpWork &w, cudaStream_t st) {
   return TT_CUDA_SUCCESS;
 }
 
+// `once`: one contraction (not a weighted sum of several scales), which
+// inside a pipeline call leaves its status to the call.
 tt_cuda_status up_alloc(const GridDims &g, bool want_acc, bool want_h,
-                        UpWork &w, int raw_passes = 0) {
+                        UpWork &w, int raw_passes = 0, bool once = false) {
   const size_t N = (size_t)g.cells();
   Workspace &ws = workspace();
   // Exits are ring pixels: at most 124 per tile.
@@ -1064,7 +1067,9 @@ tt_cuda_status up_alloc(const GridDims &g, bool want_acc, bool want_h,
                 align_up(N * 2) + align_up((size_t)g.tiles() * kRing) +
                 (size_t)raw_passes * align_up(N * 8) + 4096;
   if (!ws.reserve(need)) return TT_CUDA_ERR_ALLOC;
-  w.counters = (int *)ws.take(256);
+  int *const block = once && call_arena() ? call_arena()->block(REC_FOREST) : nullptr;
+  w.in_arena = block != nullptr;
+  w.counters = block ? block : (int *)ws.take(256);
   w.plan = (int *)ws.take(256);
   w.cell = (CoarseCell *)ws.take(N * sizeof(CoarseCell));
   w.ccell = (CoarseCell *)ws.take(E * sizeof(CoarseCell));
@@ -1088,7 +1093,7 @@ tt_cuda_status up_run(const uint8_t *dir, const float *weights, int wshift,
                       int *count_out = nullptr, long long *raw_out = nullptr,
                       const int *plan = nullptr, int pass = 0) {
   const int T = g.tiles();
-  TT_CHECK(cudaMemsetAsync(w.counters, 0, 256, st));
+  if (!w.in_arena) TT_CHECK(cudaMemsetAsync(w.counters, 0, 256, st));
   UpArgs a{};
   a.dir = dir;
   a.m = g.m;
@@ -1173,6 +1178,10 @@ tt_cuda_status up_run(const uint8_t *dir, const float *weights, int wshift,
 
 // Reads the counters back and maps error bits to a status.
 tt_cuda_status up_status(UpWork &w, cudaStream_t st, int *host6) {
+  if (w.in_arena) {  // read after the pipeline's last stage
+    for (int k = 0; k < 6; k++) host6[k] = 0;
+    return TT_CUDA_SUCCESS;
+  }
   // deferred: ecount, processed and error bits go to the status sink (when
   // the sink is full, the status is read back here as usual)
   if (int *rec = status_sink() ? sink_record(REC_FOREST, st) : nullptr) {
@@ -1381,7 +1390,7 @@ tt_cuda_status accumulate_dev(float *acc, const uint8_t *dir,
   }
   WeightPlan plan;
   TT_TRY_STATUS(weight_plan(weights, g, st, &plan));
-  TT_TRY_STATUS(up_alloc(g, true, false, w, plan.passes > 1 ? plan.passes : 0));
+  TT_TRY_STATUS(up_alloc(g, true, false, w, plan.passes > 1 ? plan.passes : 0, !weights));
   return accumulate_planned(acc, dir, weights, plan, g, false, w, st, h6);
 }
 
@@ -1389,7 +1398,7 @@ tt_cuda_status node_order_dev(ptrdiff_t *node, const uint8_t *dir,
                               const GridDims &g, unsigned order,
                               cudaStream_t st) {
   UpWork w;
-  TT_TRY_STATUS(up_alloc(g, false, true, w));
+  TT_TRY_STATUS(up_alloc(g, false, true, w, 0, true));
   TT_TRY_STATUS(up_run(dir, nullptr, 0, g, order, false, true, nullptr, w, st));
   TT_TRY_STATUS(keep_hmax(w, st));
   int h6[6];
@@ -1415,7 +1424,7 @@ tt_cuda_status node_order_acc_dev(ptrdiff_t *node, float *acc, const uint8_t *di
   } else {
     WeightPlan plan;
     TT_TRY_STATUS(weight_plan(weights, g, st, &plan));
-    TT_TRY_STATUS(up_alloc(g, true, true, w, plan.passes > 1 ? plan.passes : 0));
+    TT_TRY_STATUS(up_alloc(g, true, true, w, plan.passes > 1 ? plan.passes : 0, !weights));
     s = accumulate_planned(acc, dir, weights, plan, g, true, w, st, h6);
   }
   if (s == TT_CUDA_ERR_CYCLE) return s;

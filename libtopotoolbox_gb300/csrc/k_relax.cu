@@ -91,6 +91,10 @@ struct QueueCtl {
   int thresh;                 // ordered schedules: tiles with priority <= thresh run
 };
 
+static_assert(offsetof(QueueCtl, visits) == 0 && offsetof(QueueCtl, done) % 8 == 0 &&
+              offsetof(QueueCtl, abort) == kRelaxAbort * sizeof(int) &&
+              sizeof(QueueCtl) <= kBlockInts * sizeof(int), "status blocks hold it in place");
+
 enum : int { ABORT_SPIN = 1, ABORT_VISITS = 2 };
 
 constexpr long long kSpinLimit = 1LL << 22;  // idle scans before giving up
@@ -1151,8 +1155,16 @@ tt_cuda_status run_queue(float *state, const float *aux, const int32_t *flats,
   if (KIND != FILL && !seeded) need += align_up((size_t)g.cells() * 4);
   if (ordered) need += align_up((size_t)T * 4) + align_up((size_t)wmax * 4);
   if (!ws.reserve(need)) return TT_CUDA_ERR_ALLOC;
-  QueueCtl *ctl = (QueueCtl *)ws.take(sizeof(QueueCtl));
-  int *dirty = seeded ? seeded_dirty : (int *)ws.take((size_t)T * 4);
+  // inside a pipeline call the control block and the flags come cleared
+  CallArena *const arena = call_arena();
+  QueueCtl *ctl = (QueueCtl *)(!arena ? nullptr
+                               : report ? arena->block(REC_RELAX)
+                                        : arena->zeroed(sizeof(QueueCtl)));
+  const bool in_arena = ctl != nullptr;
+  if (!ctl) ctl = (QueueCtl *)ws.take(sizeof(QueueCtl));
+  int *dirty = seeded ? seeded_dirty : arena ? (int *)arena->zeroed((size_t)T * 4) : nullptr;
+  const bool dirty_clear = dirty != nullptr;
+  if (!dirty) dirty = (int *)ws.take((size_t)T * 4);
   // gwdt relaxes over a copy of the costs with NaN at non-flat pixels (a
   // seeded run over the costs array itself, already in that form)
   float *wcost = KIND == FILL ? nullptr
@@ -1171,10 +1183,10 @@ tt_cuda_status run_queue(float *state, const float *aux, const int32_t *flats,
   }
   const int64_t cap_rounds = max_rounds();
   ra.max_visits = (unsigned long long)T * (unsigned long long)std::min<int64_t>(cap_rounds, 1LL << 20);
-  TT_CHECK(cudaMemsetAsync(ctl, 0, sizeof(QueueCtl), st));
+  if (!in_arena) TT_CHECK(cudaMemsetAsync(ctl, 0, sizeof(QueueCtl), st));
+  if (!dirty_clear) TT_CHECK(cudaMemsetAsync(dirty, 0, (size_t)T * 4, st));
   const int tgrid = (T + 255) / 256;
   if (KIND == FILL && bc && bound) {
-    TT_CHECK(cudaMemsetAsync(dirty, 0, (size_t)T * 4, st));
     if (g.m % kCoarse == 0 && aligned16(state) && aligned16(aux) && aligned4(bc))
       TT_LAUNCH(fill_bound_init4_kernel, col_grid(g.m / kCoarse, g.n), 256, 0, st,
                 (float4 *)state, (const float4 *)aux, (const uint32_t *)bc, bound, g.m, g.n,
@@ -1185,13 +1197,11 @@ tt_cuda_status run_queue(float *state, const float *aux, const int32_t *flats,
     TT_LAUNCH(dirty_bound_kernel, tgrid, 256, 0, st, dirty, prio, bound, bound_seeds,
               bound_mc, bound_nc, g.tm, T);
   } else if (KIND == FILL && bc) {
-    TT_CHECK(cudaMemsetAsync(dirty, 0, (size_t)T * 4, st));
     TT_LAUNCH(fill_init_kernel, elementwise_grid(g.cells()), 256, 0, st, state, aux, bc, g.m,
               g.n, dirty, prio, g.tm);
   } else if (KIND == FILL) {
     TT_LAUNCH(dirty_all_kernel, tgrid, 256, 0, st, dirty, prio, T);
   } else if (!seeded) {
-    TT_CHECK(cudaMemsetAsync(dirty, 0, (size_t)T * 4, st));
     TT_LAUNCH(gwdt_init_kernel, elementwise_grid(g.cells()), 256, 0, st, state, wcost, aux,
               flats, g.m, g.n, ra);
   }
@@ -1222,6 +1232,7 @@ tt_cuda_status run_queue(float *state, const float *aux, const int32_t *flats,
     default: TT_CHECK((launch_relax<KIND, 0>(grid, ra, st))); break;
   }
   TT_CHECK(cudaGetLastError());
+  if (in_arena) return TT_CUDA_SUCCESS;  // read after the pipeline's last stage
   // deferred: the abort word goes to the status sink, no round trip (when the
   // sink is full, the status is read back here as usual)
   if (status_sink() && !report) return TT_CUDA_SUCCESS;  // an intermediate run
@@ -1251,7 +1262,7 @@ tt_cuda_status fill_impl(float *f, const float *dem, const uint8_t *bc, const Gr
   const int64_t mc = (g.m + kCoarse - 1) / kCoarse, nc = (g.n + kCoarse - 1) / kCoarse;
   const size_t Nc = (size_t)(mc * nc);
   char *buf = nullptr;
-  TT_CHECK(cudaMallocAsync((void **)&buf, align_up(Nc * 4) * 2 + align_up(Nc), st));
+  TT_CHECK(stream_alloc((void **)&buf, align_up(Nc * 4) * 2 + align_up(Nc), st));
   float *dc = (float *)buf, *fc = (float *)(buf + align_up(Nc * 4));
   uint8_t *bcc = (uint8_t *)(buf + 2 * align_up(Nc * 4));
   if (g.m % kCoarse == 0 && aligned16(dem) && aligned4(bc))
@@ -1279,7 +1290,7 @@ tt_cuda_status reconstruct_dev(float *marker, const float *mask,
   // The negated copies live in the io-independent scratch of this call.
   const int64_t N = g.cells();
   float *buf = nullptr;
-  TT_CHECK(cudaMallocAsync((void **)&buf, (size_t)N * 8, st));
+  TT_CHECK(stream_alloc((void **)&buf, (size_t)N * 8, st));
   float *f = buf, *z = buf + N;
   TT_LAUNCH(negate_pair_kernel, elementwise_grid(N), 256, 0, st, f, z, marker, mask, N);
   tt_cuda_status s = run_queue<FILL>(f, z, nullptr, g, st);

@@ -419,7 +419,7 @@ tt_cuda_status sfgraph_dev(const double *topo, size_t *rcv, double *dist, size_t
   SfScratch s;
   const size_t bytes = align_up((size_t)N) + 5 * align_up((size_t)N * 4) +
                        2 * align_up((size_t)(nb + 1) * 4) + rootward_bytes(N);
-  TT_CHECK(cudaMallocAsync((void **)&s.base, bytes, st));
+  TT_CHECK(stream_alloc((void **)&s.base, bytes, st));
   uint8_t *dir = (uint8_t *)s.take(N);
   int *parent = (int *)s.take(N * 4), *size = (int *)s.take(N * 4);
   int *val = (int *)s.take(N * 4), *rootsz = (int *)s.take(N * 4);
@@ -458,7 +458,7 @@ tt_cuda_status sf_drainage_area_dev(double *area, const size_t *rcv, int64_t row
   const ptrdiff_t dims[2] = {cols, rows};
   const GridDims g = make_dims(dims);
   SfScratch s;
-  TT_CHECK(cudaMallocAsync((void **)&s.base, 256 + align_up((size_t)N) +
+  TT_CHECK(stream_alloc((void **)&s.base, 256 + align_up((size_t)N) +
                                                  2 * align_up((size_t)N * 4), st));
   int *err = (int *)s.take(256);
   uint8_t *dir = (uint8_t *)s.take(N);

@@ -183,6 +183,7 @@ identifyflats_kernel(int32_t *__restrict__ out, const float *__restrict__ dem, i
         if (j < n) out[j * m + i] = os[cc][tx];
       }
   }
+  if (!slots) return;  // the count was not asked for
   for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
   if (tx == 0) wsum[ty] = cnt;
   __syncthreads();
@@ -695,14 +696,16 @@ tt_cuda_status identifyflats_dev(int32_t *flags, const float *dem,
                                  const GridDims &g,
                                  unsigned long long *count_dev,
                                  cudaStream_t st) {
-  Workspace &ws = workspace();
-  if (!ws.reserve(1024)) return TT_CUDA_ERR_ALLOC;
-  unsigned long long *slots = (unsigned long long *)ws.take(kCountSlots * 8);
-  unsigned long long *cnt = count_dev ? count_dev : (unsigned long long *)ws.take(8);
-  TT_CHECK(cudaMemsetAsync(slots, 0, kCountSlots * 8, st));
+  unsigned long long *slots = nullptr;
+  if (count_dev) {
+    Workspace &ws = workspace();
+    if (!ws.reserve(1024)) return TT_CUDA_ERR_ALLOC;
+    slots = (unsigned long long *)ws.take(kCountSlots * 8);
+    TT_CHECK(cudaMemsetAsync(slots, 0, kCountSlots * 8, st));
+  }
   TT_LAUNCH(identifyflats_kernel, tile_grid(g), dim3(kBlockX, kBlockY), 0, st, flags, dem, g.m,
             g.n, slots);
-  TT_LAUNCH(sum_slots_kernel, 1, 32, 0, st, slots, cnt);
+  if (count_dev) TT_LAUNCH(sum_slots_kernel, 1, 32, 0, st, slots, count_dev);
   TT_CHECK(cudaGetLastError());
   return TT_CUDA_SUCCESS;
 }

@@ -125,6 +125,7 @@ class Workspace {
 // kRecordInts ints: {kind, a, b, c}.
 constexpr int kRecordInts = 4;
 enum : int { REC_RELAX = 1, REC_FOREST = 2 };
+constexpr int kRelaxAbort = 5;  // int of a relaxation's control block: its abort word
 struct StatusSink {
   int *dev;      // device array of records
   int capacity;  // records
@@ -153,6 +154,54 @@ class SinkScope {
   StatusSink *sink_;
   Workspace *ws_, *io_;
 };
+
+// Scratch of one whole pipeline call that has to start at zero: the status
+// blocks and tile flags of its stages lie together, one memset clears them,
+// and the status is read from the blocks once, after the last stage, instead
+// of after each (a 512^2 pipeline spent half its time on those round trips,
+// on a clear per stage and on allocations: 951 -> 653 us).  Stages that find
+// no arena, or a full one, clear scratch of their own and report by
+// themselves.
+constexpr int kBlockInts = 64;  // one status block
+constexpr int kArenaBlocks = 8;
+class CallArena {
+ public:
+  // Bytes of an arena for grids of `tiles` tiles.
+  static size_t bytes(int tiles);
+  // Takes `base` (bytes(tiles) long) and clears it on `st`.
+  tt_cuda_status init(void *base, int tiles, cudaStream_t st);
+  // A cleared status block for a stage of this kind (REC_*), or nullptr.
+  int *block(int kind);
+  // Cleared scratch, or nullptr when the arena is used up.
+  void *zeroed(size_t bytes);
+  // The stages' status after the last one: read back with one
+  // synchronisation, or left in the status sink when one is set.
+  tt_cuda_status collect(int tiles, cudaStream_t st);
+
+ private:
+  char *base_ = nullptr;
+  size_t used_ = 0, cap_ = 0;
+  int blocks_ = 0;
+  int kind_[kArenaBlocks] = {};
+};
+CallArena *call_arena();  // of this thread's pipeline call, or nullptr
+class ArenaScope {        // sets it for the life of the scope
+ public:
+  explicit ArenaScope(CallArena *a);
+  ~ArenaScope();
+  ArenaScope(const ArenaScope &) = delete;
+  ArenaScope &operator=(const ArenaScope &) = delete;
+
+ private:
+  CallArena *prev_;
+};
+
+// Stream-ordered device memory of one call, from a pool of this library per
+// device.  It keeps up to kPoolKeep bytes when they are freed: the default
+// pool gives everything back at each synchronisation, and mapping it again
+// took 100 us a call.  tt_cuda_release_workspace gives it back.
+constexpr size_t kPoolKeep = (size_t)256 << 20;
+cudaError_t stream_alloc(void **p, size_t bytes, cudaStream_t st);
 
 Workspace &workspace();          // of the current device (or the override)
 void *pinned_scratch();          // 4 KiB of pinned host memory per device

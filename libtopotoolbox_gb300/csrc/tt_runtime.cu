@@ -19,6 +19,7 @@ thread_local int64_t g_last_rounds = 0;
 thread_local StatusSink *g_sink = nullptr;
 thread_local Workspace *g_ws_override = nullptr;
 thread_local Workspace *g_io_override = nullptr;
+thread_local CallArena *g_arena = nullptr;
 thread_local int g_relax_schedule = -1;  // -1: the environment's or 0
 int64_t g_max_rounds_override = 0;
 
@@ -30,6 +31,7 @@ struct DeviceState {
   Workspace scratch;
   Workspace io;
   void *pinned = nullptr;
+  cudaMemPool_t pool = nullptr;
   int sms = 0;
   // side streams and events for host-device copies that overlap the
   // kernels of a host-pointer call
@@ -120,6 +122,112 @@ int *sink_record(int kind, cudaStream_t st) {
   cudaMemsetAsync(rec, 0, kRecordInts * sizeof(int), st);
   cudaMemsetAsync(rec, kind, 1, st);
   return rec;
+}
+
+CallArena *call_arena() { return g_arena; }
+ArenaScope::ArenaScope(CallArena *a) : prev_(g_arena) { g_arena = a; }
+ArenaScope::~ArenaScope() { g_arena = prev_; }
+
+constexpr size_t kBlockBytes = kBlockInts * sizeof(int);
+
+size_t CallArena::bytes(int tiles) {
+  // tile flags of the fill, of its coarser starts and of gwdt
+  return kArenaBlocks * kBlockBytes + 3 * (align_up((size_t)tiles * 4) + 1024);
+}
+
+tt_cuda_status CallArena::init(void *base, int tiles, cudaStream_t st) {
+  base_ = (char *)base;
+  cap_ = bytes(tiles);
+  used_ = kArenaBlocks * kBlockBytes;
+  blocks_ = 0;
+  TT_CHECK(cudaMemsetAsync(base_, 0, cap_, st));
+  return TT_CUDA_SUCCESS;
+}
+
+int *CallArena::block(int kind) {
+  if (blocks_ == kArenaBlocks) return nullptr;
+  kind_[blocks_] = kind;
+  return (int *)(base_ + (size_t)blocks_++ * kBlockBytes);
+}
+
+void *CallArena::zeroed(size_t bytes) {
+  if (used_ + align_up(bytes) > cap_) return nullptr;
+  void *p = base_ + used_;
+  used_ += align_up(bytes);
+  return p;
+}
+
+namespace {
+// The record {kind, a, b, c} of a stage's status block: a relaxation's abort
+// word, or a forest's exit count, exits processed and error bits.
+__host__ __device__ void block_record(int kind, const int *block, int *rec) {
+  rec[0] = kind;
+  rec[1] = kind == REC_RELAX ? block[kRelaxAbort] : block[0];
+  rec[2] = kind == REC_RELAX ? 0 : block[2];
+  rec[3] = kind == REC_RELAX ? 0 : block[4];
+}
+
+struct BlockKinds {
+  int kind[kArenaBlocks];
+};
+
+__global__ void collect_blocks_kernel(const int *__restrict__ blocks, BlockKinds kinds,
+                                      int count, int *__restrict__ rec) {
+  const int k = threadIdx.x;
+  if (k < count) block_record(kinds.kind[k], blocks + k * kBlockInts, rec + k * kRecordInts);
+}
+}  // namespace
+
+tt_cuda_status CallArena::collect(int tiles, cudaStream_t st) {
+  if (!blocks_) return TT_CUDA_SUCCESS;
+  StatusSink *sink = status_sink();
+  if (sink && sink->next + blocks_ <= sink->capacity) {
+    BlockKinds kinds;
+    std::memcpy(kinds.kind, kind_, sizeof(kind_));
+    TT_LAUNCH(collect_blocks_kernel, 1, 32, 0, st, (const int *)base_, kinds, blocks_,
+              sink->dev + (size_t)sink->next * kRecordInts);
+    sink->next += blocks_;
+    TT_CHECK(cudaGetLastError());
+    return TT_CUDA_SUCCESS;
+  }
+  int *h = (int *)pinned_scratch();
+  if (!h) return TT_CUDA_ERR_ALLOC;
+  TT_CHECK(cudaMemcpyAsync(h, base_, (size_t)blocks_ * kBlockBytes, cudaMemcpyDeviceToHost, st));
+  TT_CHECK(cudaStreamSynchronize(st));
+  tt_cuda_status s = TT_CUDA_SUCCESS;
+  for (int k = 0; k < blocks_; k++) {  // the last failure, as stage by stage
+    const int *b = h + k * kBlockInts;
+    int rec[kRecordInts];
+    block_record(kind_[k], b, rec);
+    const tt_cuda_status r = sink_status(rec, 1);
+    if (r != TT_CUDA_SUCCESS) s = r;
+    if (kind_[k] == REC_RELAX && !sink) {
+      unsigned long long visits;
+      std::memcpy(&visits, b, 8);
+      set_last_rounds((int64_t)(visits / (unsigned long long)(tiles > 0 ? tiles : 1)));
+    }
+  }
+  return s;
+}
+
+cudaError_t stream_alloc(void **p, size_t bytes, cudaStream_t st) {
+  const int dev = current_device();
+  DeviceState &d = g_dev[dev];
+  if (!d.pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    uint64_t keep = kPoolKeep;
+    if (cudaMemPoolCreate(&d.pool, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      cudaGetLastError();
+      if (d.pool) cudaMemPoolDestroy(d.pool);
+      d.pool = nullptr;
+      return cudaMallocAsync(p, bytes, st);
+    }
+  }
+  return cudaMallocFromPoolAsync(p, bytes, d.pool, st);
 }
 
 bool cuda_ok(cudaError_t e, const char *what) {
@@ -330,6 +438,7 @@ void tt_cuda_release_workspace(void) {
   DeviceLock lock;
   workspace().release();
   io_workspace().release();
+  if (cudaMemPool_t pool = g_dev[current_device()].pool) cudaMemPoolTrimTo(pool, 0);
   if (g_defer && !g_defer->active) release_deferral(*g_defer);
 }
 
@@ -775,10 +884,15 @@ static tt_cuda_status pipeline_body(float *filled, int32_t *flats, float *dist,
                                     const uint8_t *bc, const float *weights,
                                     float az, float alt, float cs,
                                     float *costs, ptrdiff_t *conncomps,
-                                    const GridDims &g, cudaStream_t st,
-                                    EarlyOut *out = nullptr) {
+                                    void *arena_base, const GridDims &g,
+                                    cudaStream_t st, EarlyOut *out = nullptr) {
   tt_cuda_status soft = TT_CUDA_SUCCESS;
   const size_t n = (size_t)g.m * (size_t)g.n;
+  CallArena arena;
+  ArenaScope scope(&arena);
+  TT_TRY(arena.init(arena_base, g.tiles(), st));
+  // gwdt's tile flags, when the costs pass writes its start (below)
+  int *const gdirty = relax_schedule() < 4 ? (int *)arena.zeroed((size_t)g.tiles() * 4) : nullptr;
   TT_TRY_SOFT(fill_dev(filled, dem, bc, g, st), soft);
   if (out) TT_TRY(out->send(out->filled, filled, n * 4, st));
   TT_TRY(identifyflats_dev(flats, filled, g, nullptr, st));
@@ -786,16 +900,7 @@ static tt_cuda_status pipeline_body(float *filled, int32_t *flats, float *dist,
   // The costs pass writes the gwdt start directly (the pipeline does not
   // return the costs), except under the ordered schedules, whose tile
   // priorities the start would have to set as well.
-  if (relax_schedule() < 4) {
-    const size_t tb = (size_t)g.tiles() * 4;
-    int *gdirty = nullptr;
-    TT_CHECK(cudaMallocAsync((void **)&gdirty, tb, st));
-    struct Free {
-      void *p;
-      cudaStream_t st;
-      ~Free() { cudaFreeAsync(p, st); }
-    } free_dirty{gdirty, st};
-    TT_CHECK(cudaMemsetAsync(gdirty, 0, tb, st));
+  if (gdirty) {
     const GwdtSeed seed{dist, gdirty};
     TT_TRY(costs_dev(costs, conncomps, flats, dem, filled, g, st, &seed));
     TT_TRY_SOFT(gwdt_seeded_dev(dist, costs, flats, gdirty, g, st), soft);
@@ -831,6 +936,7 @@ static tt_cuda_status pipeline_body(float *filled, int32_t *flats, float *dist,
     if (out && acc) TT_TRY(out->send(out->acc, acc, n * 4, st));
   }
   if (hill) TT_TRY(hillshade_dev(hill, dem, az, alt, cs, g, st));
+  TT_TRY_SOFT(arena.collect(g.tiles(), st), soft);
   if (out) TT_TRY(out->join(st));
   return soft;
 }
@@ -851,15 +957,17 @@ extern "C" tt_cuda_status tt_cuda_d8_pipeline_dev(
     if (!flats) sg.add(N * 4);
     if (!dist) sg.add(N * 4);
     if (!direction) sg.add(N);
+    sg.add(CallArena::bytes(g.tiles()));
     if (!sg.reserve()) return TT_CUDA_ERR_ALLOC;
     float *costs = (float *)sg.take(N * 4);
+    void *arena = sg.take(CallArena::bytes(g.tiles()));
     if (!filled) filled = (float *)sg.take(N * 4);
     if (!flats) flats = (int32_t *)sg.take(N * 4);
     if (!dist) dist = (float *)sg.take(N * 4);
     if (!direction) direction = (uint8_t *)sg.take(N);
     return pipeline_body(filled, flats, dist, node, direction, acc, hillshade,
                          dem, bc, weights, azimuth, altitude, cellsize, costs,
-                         nullptr, g, st);
+                         nullptr, arena, g, st);
   });
 }
 
@@ -1187,7 +1295,7 @@ void host_edge_sweep(V *output, const V *input, const ptrdiff_t *source,
   if (s == TT_CUDA_SUCCESS && N >= (1LL << 31)) s = TT_CUDA_ERR_INVALID_ARGUMENT;
   V *dout = nullptr;
   if (s == TT_CUDA_SUCCESS &&
-      cudaMallocAsync((void **)&dout, (size_t)N * sizeof(V), st) != cudaSuccess) {
+      stream_alloc((void **)&dout, (size_t)N * sizeof(V), st) != cudaSuccess) {
     cudaGetLastError();
     s = TT_CUDA_ERR_ALLOC;
     dout = nullptr;
@@ -1380,7 +1488,9 @@ void tt_cuda_d8_pipeline(float *filled, int32_t *flats, float *dist,
              {nullptr, node ? N * 8 : 0, false, false},
              {nullptr, N, false, false},
              {nullptr, acc ? N * 4 : 0, false, false},
-             {nullptr, N * 4, false, false}},  // costs
+             {nullptr, N * 4, false, false},  // costs
+             {nullptr, dims_ok(dims) ? CallArena::bytes(make_dims(dims).tiles()) : 0, false,
+              false}},
             [&](const GridDims &g, cudaStream_t st, std::vector<HostArg> &a) {
               EarlyOut out;
               out.filled = filled;
@@ -1395,7 +1505,7 @@ void tt_cuda_d8_pipeline(float *filled, int32_t *flats, float *dist,
                   node ? (ptrdiff_t *)a[6].dev : nullptr, (uint8_t *)a[7].dev,
                   acc ? (float *)a[8].dev : nullptr, nullptr, (const float *)a[0].dev,
                   (const uint8_t *)a[1].dev, weights ? (const float *)a[2].dev : nullptr,
-                  0.f, 0.f, 1.f, (float *)a[9].dev, nullptr, g, st, &out);
+                  0.f, 0.f, 1.f, (float *)a[9].dev, nullptr, a[10].dev, g, st, &out);
               // copies already issued end before the call returns, even when
               // a later stage failed
               if (out.cs && out.used && cudaStreamSynchronize(out.cs) != cudaSuccess) {
