@@ -567,11 +567,12 @@ __device__ __forceinline__ void cas128(CoarseCell *p, unsigned long long &lo,
 
 // Last-arriver walk over the exits: a walker owns a complete exit, folds its
 // totals into the next exit downstream with one compare-and-swap, and
-// continues only if it was the last donor to arrive.  The next exit's link
-// is loaded together with its cell, so a hop costs two dependent accesses;
-// into an exit with a single coarse donor (most hops along a river) the
-// walker is the only arrival, so it combines and stores without the swap:
-// one dependent access per hop.
+// continues only if it was the last donor to arrive.  Into an exit with a
+// single coarse donor the walker is the only arrival, so it combines and
+// stores without the swap.  The longest chain of hops bounds the walk, so
+// the link and cell of the exit after the next are read while this hop's
+// swap is under way (a cell that changes meanwhile only makes its swap
+// fail and return the new value): one dependent access a hop.
 __global__ void coarse_walk_kernel(const int *__restrict__ leaves,
                                    const int *__restrict__ lcount,
                                    const int2 *__restrict__ link,
@@ -585,38 +586,47 @@ __global__ void coarse_walk_kernel(const int *__restrict__ leaves,
     long long v = c0.x;
     int hv = (int)(unsigned)(unsigned long long)c0.y;
     int2 l = link[e0];
+    n_done++;
+    if (l.x < 0) continue;
+    longlong2 g = __ldcg(reinterpret_cast<const longlong2 *>(&ccell[l.x]));
+    int2 ln = link[l.x];
     for (int guard = 0; guard < limit; guard++) {
-      n_done++;
       const int nx = l.x;
-      if (nx < 0) break;
-      const longlong2 g = __ldcg(reinterpret_cast<const longlong2 *>(&ccell[nx]));
-      const int2 ln = link[nx];
+      // the exit after the next one, read ahead
+      const int n2 = ln.x;
+      longlong2 g2 = {};
+      int2 l2 = {};
+      if (n2 >= 0) {
+        g2 = __ldcg(reinterpret_cast<const longlong2 *>(&ccell[n2]));
+        l2 = link[n2];
+      }
       const int hops = l.y & 0xffff;
       if ((ln.y >> 16) == 1) {  // the only coarse donor of nx: no other writer
-        const long long sum = g.x + v;
-        const int h = max((int)(unsigned)(unsigned long long)g.y, hv + hops);
+        v += g.x;
+        hv = max((int)(unsigned)(unsigned long long)g.y, hv + hops);
         __stcg(reinterpret_cast<longlong2 *>(&ccell[nx]),
-               make_longlong2(sum, (long long)(unsigned long long)(unsigned)h));
-        v = sum;
-        hv = h;
-        l = ln;
-        continue;
+               make_longlong2(v, (long long)(unsigned long long)(unsigned)hv));
+      } else {
+        unsigned long long lo = (unsigned long long)g.x, hi = (unsigned long long)g.y;
+        unsigned long long nlo, nhi;
+        for (;;) {
+          const int oh = (int)(unsigned)hi, op = (int)(unsigned)(hi >> 32);
+          nlo = lo + (unsigned long long)v;
+          nhi = (unsigned long long)(unsigned)max(oh, hv + hops) |
+                ((unsigned long long)(unsigned)(op - 1) << 32);
+          const unsigned long long elo = lo, ehi = hi;
+          cas128(&ccell[nx], lo, hi, nlo, nhi);
+          if (lo == elo && hi == ehi) break;  // swapped
+        }
+        if ((int)(unsigned)(hi >> 32) != 1) break;  // other donors still to come
+        v = (long long)nlo;  // every donor of nx has arrived: its totals are final
+        hv = (int)(unsigned)nhi;
       }
-      unsigned long long lo = (unsigned long long)g.x, hi = (unsigned long long)g.y;
-      unsigned long long nlo, nhi;
-      for (;;) {
-        const int oh = (int)(unsigned)hi, op = (int)(unsigned)(hi >> 32);
-        nlo = lo + (unsigned long long)v;
-        nhi = (unsigned long long)(unsigned)max(oh, hv + hops) |
-              ((unsigned long long)(unsigned)(op - 1) << 32);
-        const unsigned long long elo = lo, ehi = hi;
-        cas128(&ccell[nx], lo, hi, nlo, nhi);
-        if (lo == elo && hi == ehi) break;  // swapped
-      }
-      if ((int)(unsigned)(hi >> 32) != 1) break;  // other donors still to come
-      v = (long long)nlo;  // every donor of nx has arrived: its totals are final
-      hv = (int)(unsigned)nhi;
+      n_done++;
+      if (n2 < 0) break;
       l = ln;
+      ln = l2;
+      g = g2;
     }
   }
   // One atomic per warp on the shared count, not one per leaf.
