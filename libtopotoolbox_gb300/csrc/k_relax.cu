@@ -36,13 +36,16 @@
 // Termination: only a running warp sets flags.  A warp that finds none of
 // its tiles dirty adds itself to an idle count (after its own flags are
 // visible); a warp that finds a flag again leaves the count, and bumps a
-// wake counter kept in the same 64-bit word, before it takes the flag.  The
-// warp whose arrival makes every warp idle scans all flags and ends the run
-// if none is set and the word is unchanged since its arrival (no warp woke,
-// so none ran and none could set a flag behind the scan); otherwise the
-// owners of the set flags wake up and the last one to go idle scans again.  Every wait is bounded: a warp that idles too
-// long, or a run that exceeds its visit budget, raises an abort flag and all
-// warps return with an error status.
+// wake counter kept in the same 64-bit word, before the visit takes the flag
+// down at its end.  When warp 0 is idle and reads that every warp is, it
+// scans all flags and ends the run if none is set and the word is unchanged
+// since it was read (no warp woke, so none ran and none could set a flag
+// behind the scan); otherwise the owners of the set flags wake up.  Neither
+// a warp that goes idle nor one that wakes waits for its atomics: a chain of
+// visits across tiles that wait for each other crosses no more round trips
+// than the publication and one poll.  Every wait is bounded: a warp that
+// idles too long, or a run that exceeds its visit budget, raises an abort
+// flag and all warps return with an error status.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -57,11 +60,13 @@ constexpr int kWarps = 4;        // tiles per block
 constexpr int kMaxSweeps = 256;  // per tile visit; a capped tile re-enqueues
 // Tiles a warp relaxes before it looks at its flags again from its lowest
 // tile on.  Few keep the warps together in one region of a large grid, whose
-// tiles are still in L2 when they are visited again; with one, a region is
-// relaxed too far on what it knows and visited more often.  16384^2, fill /
-// gwdt ms: all 32 of a poll 8.2 / 12.1, one 6.9 / 10.4, two 6.7 / 9.8, four
-// 6.9 / 9.5 (4096^2: 1.49 / 2.30, 1.45 / 2.10, 1.44 / 2.15, 1.43 / 2.14).
-constexpr int kTakeTiles = 4;
+// tiles are still in L2 when they are visited again; too few, and a region is
+// relaxed too far on what it knows and visited more often.  16384^2: fill
+// 8.2 ms with all 32 of a poll, 6.4 with four, 6.1 with two, 6.4 with one;
+// gwdt 12.1 with all, 10.3 with 16, 10.1 with eight, 9.9 with four, 10.6
+// with two.
+constexpr int kTakeFill = 2, kTakeGwdt = 4;
+
 constexpr float kSqrt2 = 1.41421356237309504880f;
 
 // GWDT_HALF: gwdt over costs stored halved (the pipeline's own costs, at
@@ -81,17 +86,16 @@ struct WarpTile {
 };
 static_assert(sizeof(WarpTile) == (2 * kHalo + 2) * kPitch * sizeof(float), "packed rows");
 
-// Control block (device memory, zero-initialised).
-struct QueueCtl {
-  unsigned long long visits;  // tiles relaxed so far (flushed in batches)
+// Control block (device memory, zero-initialised).  Every poll reads its
+// first 16 bytes with one load.
+struct __align__(16) QueueCtl {
   unsigned long long idle;    // wakes << 32 | warps that found nothing to do
-  // done and abort are polled with one 8-byte load
   int done;                   // set once every warp is idle and no flag is set
   int abort;                  // ABORT_* bits
+  unsigned long long visits;  // tiles relaxed so far (flushed in batches)
   int thresh;                 // ordered schedules: tiles with priority <= thresh run
 };
-
-static_assert(offsetof(QueueCtl, visits) == 0 && offsetof(QueueCtl, done) % 8 == 0 &&
+static_assert(offsetof(QueueCtl, visits) == kRelaxVisits * sizeof(int) &&
               offsetof(QueueCtl, abort) == kRelaxAbort * sizeof(int) &&
               sizeof(QueueCtl) <= kBlockInts * sizeof(int), "status blocks hold it in place");
 
@@ -125,8 +129,13 @@ __device__ __forceinline__ float key_value(int k) {
 constexpr int kClean = 0x7f7f7f7f;        // no priority (above every finite key)
 constexpr int kUrgent = (int)0x80000000;  // below every key: runs at any threshold
 
-// Dirty flag bits: 1 = a halo pixel changed (re-evaluate the edge ring),
-// 2 = evaluate every pixel (first visit, or a visit that hit its sweep cap).
+// A tile's dirty word counts the changes published to it that it has not
+// taken in yet: DIRTY_EDGE for each time a neighbour lowers a pixel of its
+// halo (evaluate the edge ring), DIRTY_FULL to have every pixel evaluated
+// (first visit, or a visit that hit its sweep cap).  The owner subtracts
+// what it read when the visit that took it in is over, so a change published
+// meanwhile keeps the word set, no exchange has to come back before a visit
+// can begin, and the word of a tile in work is never zero.
 
 // Release / acquire at device scope (lighter than a sequentially consistent
 // fence): a writer fences before it sets a flag, a reader after it takes one.
@@ -190,8 +199,8 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 //
 // The sweeps took 177 cycles a step on an idle SM and 291 (fill) to 380
 // (gwdt) on a busy one with a branch around the store, a barrier and the
-// loads of the same step on the chain; in the form below they take 82 and
-// 179 to 222 (16384^2 gwdt 13.4 -> 12.2 ms, 4096^2 3.4 -> 2.4 ms).
+// loads of the same step on the chain; in the form below they take 67 and
+// 179 to 222.
 //
 // What bounds a sweep is the chain from one step's results to the next
 // step's inputs, on small grids and at the end of every run, and the issue
@@ -202,10 +211,13 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 // everything else, and the centre's own update.  All other operands are
 // read from shared memory one step ahead, results are stored without being
 // read again in the same sweep (no barrier between steps), and the changed
-// bits are shifted into a mask.  Sweeps start at the group of kSweepUnroll
+// bits are shifted into a mask.  Sweeps start at the group of unrolled
 // steps that holds the first marked one (evaluating an unmarked pixel
-// changes nothing).
-constexpr int kSweepUnroll = 4;
+// changes nothing).  Unrolling spares the moves between the rows' registers
+// and costs instruction cache, which the four copies of a sweep share:
+// 16384^2 fill 6.12 ms unrolled four times, 6.00 eight, 6.94 sixteen; gwdt
+// 10.8 ms unrolled twice, 9.9 four times, 13.2 eight.
+constexpr int kUnrollFill = 8, kUnrollGwdt = 4;
 
 __device__ __forceinline__ void remark(int lane, int first, int dir, uint32_t dm, uint32_t &nd,
                                        uint32_t &dm_all) {
@@ -222,10 +234,11 @@ __device__ __forceinline__ void remark(int lane, int first, int dir, uint32_t dm
 }
 
 // First step of a sweep over the marks `nd` (32: nothing marked).
+template <int UNROLL>
 __device__ __forceinline__ int first_step(uint32_t nd, int dir) {
   const uint32_t steps = __reduce_or_sync(0xffffffffu, nd);
   if (!steps) return kTile;
-  return (dir > 0 ? __ffs(steps) - 1 : __clz(steps)) & ~(kSweepUnroll - 1);
+  return (dir > 0 ? __ffs(steps) - 1 : __clz(steps)) & ~(UNROLL - 1);
 }
 
 // chamfer * (c(u) + c(v)) / 2 between side and corner neighbours;
@@ -246,7 +259,7 @@ __device__ __forceinline__ float diag_weight(float c, float d) {
 template <bool ALONG_C, int DIR>
 __device__ __forceinline__ void sweep_fill(WarpTile &t, int lane, uint32_t &nd,
                                            uint32_t &dm_all) {
-  const int first = first_step(nd, DIR);
+  const int first = first_step<kUnrollFill>(nd, DIR);
   if (first >= kTile) return;
   // Pixel (line l, position p): t.s[l][p] in the column layout, t.s[p][l]
   // in the row layout.  The lane's line is l = lane + 1.
@@ -265,16 +278,19 @@ __device__ __forceinline__ void sweep_fill(WarpTile &t, int lane, uint32_t &nd,
   float lp = sp[-LS], op = sp[0], rp = sp[LS], z = ap[0];  // here
   float la = sp[-LS + D], oa = sp[D], ra = sp[LS + D];     // ahead
 #pragma unroll 1
-  for (int s = first; s < kTile; s += kSweepUnroll) {
+  for (int s = first; s < kTile; s += kUnrollFill) {
 #pragma unroll
-    for (int u = 0; u < kSweepUnroll; u++) {
+    for (int u = 0; u < kUnrollFill; u++) {
       // the next step's row ahead and centre (the last step reads past the
       // halo, inside the tile arrays, and its values are not used)
       const float la2 = sp[-LS + 2 * D], oa2 = sp[2 * D], ra2 = sp[LS + 2 * D], z2 = ap[D];
       const float ls = __shfl_up_sync(0xffffffffu, ob, 1);
       const float rs = __shfl_down_sync(0xffffffffu, ob, 1);
-      const float pre = min3(min3(op, lp, rp), min3(la, oa, ra), ob);
-      const float nv = max_nan(z, min3(pre, lo_lane ? lh : ls, hi_lane ? rh : rs));
+      // the outer lanes get their own value back by the shuffle (it is in
+      // the minimum anyway) and the halo line's value here
+      const float edge = lo_lane ? lh : hi_lane ? rh : ra;
+      const float pre = min3(min3(op, lp, rp), min3(la, oa, ra), fminf(ob, edge));
+      const float nv = max_nan(z, min3(pre, ls, rs));
       const bool ch = nv < op;
       if (ch) sp[0] = nv;
       dm = dm + dm + (ch ? 1u : 0u);
@@ -304,7 +320,7 @@ __device__ __forceinline__ void sweep_fill(WarpTile &t, int lane, uint32_t &nd,
 template <bool ALONG_C, int DIR, bool HALF>
 __device__ __forceinline__ void sweep_gwdt(WarpTile &t, int lane, uint32_t &nd,
                                            uint32_t &dm_all) {
-  const int first = first_step(nd, DIR);
+  const int first = first_step<kUnrollGwdt>(nd, DIR);
   if (first >= kTile) return;
   constexpr int PS = ALONG_C ? kPitch : 1;
   constexpr int LS = ALONG_C ? 1 : kPitch;
@@ -326,9 +342,9 @@ __device__ __forceinline__ void sweep_gwdt(WarpTile &t, int lane, uint32_t &nd,
   float ca0 = ap[-LS + D], ca1 = ap[D], ca2 = ap[LS + D];
   float wb = side(cp1, ap[-D]);  // own line: between behind and here
 #pragma unroll 1
-  for (int s = first; s < kTile; s += kSweepUnroll) {
+  for (int s = first; s < kTile; s += kUnrollGwdt) {
 #pragma unroll
-    for (int u = 0; u < kSweepUnroll; u++) {
+    for (int u = 0; u < kUnrollGwdt; u++) {
       const float la2 = sp[-LS + 2 * D], oa2 = sp[2 * D], ra2 = sp[LS + 2 * D];
       const float d0 = ap[-LS + 2 * D], d1 = ap[2 * D], d2 = ap[LS + 2 * D];
       const float ls = __shfl_up_sync(0xffffffffu, ob, 1);
@@ -377,21 +393,29 @@ __device__ __forceinline__ void sweep(WarpTile &t, int lane, uint32_t &nd, uint3
     sweep_gwdt<ALONG_C, DIR, KIND == GWDT_HALF>(t, lane, nd, dm_all);
 }
 
-// Whether the tile's values would lower the halo pixel at word `q` of the
+// Whether the tile's own values lower the halo pixel at word `q` of the
 // tile: `n` is the pixel of the tile beside it, `along` the stride along the
 // edge (the three pixels n - along, n, n + along touch q), 0 for a corner of
-// the halo (n alone touches it).
+// the halo (n alone touches it).  The fill, which goes on after publishing,
+// lowers it here too, as the neighbour that owns it will.
 template <int KIND>
-__device__ __forceinline__ bool lowers(const WarpTile &t, int q, int n, int along) {
-  const float *const s = reinterpret_cast<const float *>(&t);
+__device__ __forceinline__ bool lower(WarpTile &t, int q, int n, int along) {
+  float *const s = reinterpret_cast<float *>(&t);
   const float *const a = s + kHalo * kPitch;
   constexpr bool HALF = KIND == GWDT_HALF;
+  float v;
   if (KIND == FILL)
-    return max_nan(a[q], along ? min3(s[n - along], s[n], s[n + along]) : s[n]) < s[q];
-  if (!along) return __fadd_rn(s[n], diag_weight<HALF>(a[q], a[n])) < s[q];
-  return min3(__fadd_rn(s[n - along], diag_weight<HALF>(a[q], a[n - along])),
-              __fadd_rn(s[n], side_weight<HALF>(a[q], a[n])),
-              __fadd_rn(s[n + along], diag_weight<HALF>(a[q], a[n + along]))) < s[q];
+    v = max_nan(a[q], along ? min3(s[n - along], s[n], s[n + along]) : s[n]);
+  else if (!along)
+    v = __fadd_rn(s[n], diag_weight<HALF>(a[q], a[n]));
+  else
+    v = min3(__fadd_rn(s[n - along], diag_weight<HALF>(a[q], a[n - along])),
+             __fadd_rn(s[n], side_weight<HALF>(a[q], a[n])),
+             __fadd_rn(s[n + along], diag_weight<HALF>(a[q], a[n + along])));
+  if (KIND != FILL) return v < s[q];
+  if (!(v < s[q])) return false;
+  s[q] = v;
+  return true;
 }
 
 // Sweep schedules (a template parameter, picked at run time): bit 0 runs the
@@ -419,7 +443,7 @@ __device__ __forceinline__ int band_above(int key, int sched) {
 }
 
 template <int KIND, int SCHED>
-__device__ void relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, int mode);
+__device__ bool relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, int mode);
 
 // Ordered schedules: with every warp idle, raise the threshold above the
 // lowest priority any warp reported waiting.  Returns false when no warp
@@ -435,9 +459,11 @@ __device__ bool raise_threshold(const RelaxArgs &a, int lane, int W, int thr) {
   return true;
 }
 
-// The warp that made every warp idle (idle word `seen` after its arrival):
-// finish the run if no flag is set and no warp has woken since.
+// With every warp idle (idle word `seen`): finish the run if no flag is set
+// and no warp has woken since.  A warp leaves the idle count before it takes
+// a word down, so a flag that is gone shows in the count.
 __device__ void check_done(const RelaxArgs &a, int lane, int T, unsigned long long seen) {
+  fence_acq_rel_gpu();  // every flag set before its warp went idle is visible
   bool any = false;
   for (int t = lane; t < T; t += 32) any |= *(volatile int *)&a.dirty[t] != 0;
   if (__any_sync(0xffffffffu, any) || lane != 0) return;
@@ -446,7 +472,7 @@ __device__ void check_done(const RelaxArgs &a, int lane, int T, unsigned long lo
 }
 
 template <int KIND, int SCHED>
-__global__ void __launch_bounds__(kWarps * 32)
+__global__ void __launch_bounds__(kWarps * 32, 5)
 relax_persistent_kernel(RelaxArgs a) {
   __shared__ WarpTile tiles[kWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -454,17 +480,20 @@ relax_persistent_kernel(RelaxArgs a) {
   const int W = gridDim.x * kWarps;
   const int wid = blockIdx.x * kWarps + warp;
   const int T = a.tm * a.tn;
+  constexpr int kTakeTiles = KIND == FILL ? kTakeFill : kTakeGwdt;
   long long spins = 0;
   bool idle = false;                 // counted in ctl->idle (warp-uniform)
-  unsigned long long unflushed = 0;  // lane 0: visits not yet added to ctl
+  unsigned long long unflushed = 0;  // visits not yet added to ctl
   int posted = kClean;               // ordered: this warp's last wmin entry
   int raised_at = kUrgent;           // ordered: threshold this warp last raised from
   for (;;) {
-    // The stop word and the first flags are loaded together: a poll costs
-    // one round trip to L2, which is on the path of every change that
+    // The control words and the first flags are loaded together: a poll
+    // costs one round trip to L2, which is on the path of every change that
     // crosses tiles.
-    const unsigned long long stop_word = *(volatile unsigned long long *)&a.ctl->done;
-    int f0 = wid + lane * W < T ? *(volatile int *)&a.dirty[wid + lane * W] : 0;
+    unsigned long long idle_word, stop_word;
+    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];"
+                 : "=l"(idle_word), "=l"(stop_word) : "l"(a.ctl) : "memory");
+    const int f0 = wid + lane * W < T ? *(volatile int *)&a.dirty[wid + lane * W] : 0;
     const int thr = ordered_sched(SCHED) ? *(volatile int *)&a.ctl->thresh : 0;
     if (stop_word) break;
     int lane_wait = kClean;  // ordered: lowest priority of this lane's waiting tiles
@@ -473,9 +502,8 @@ relax_persistent_kernel(RelaxArgs a) {
         atomicOr(&a.ctl->abort, ABORT_VISITS);
       unflushed = 0;
     }
-    bool did = false;
     int taken = 0;
-    for (int base = wid; base < T; base += W * 32) {
+    for (int base = wid; base < T && taken < kTakeTiles; base += W * 32) {
       const int mine = base + lane * W;
       int f = f0;
       if (base != wid) f = (mine < T) ? *(volatile int *)&a.dirty[mine] : 0;
@@ -488,38 +516,32 @@ relax_persistent_kernel(RelaxArgs a) {
         if (!elig) lane_wait = min(lane_wait, pr == kClean ? kClean - 1 : pr);
       }
       unsigned mask = __ballot_sync(0xffffffffu, elig);
-      if (mask && idle) {  // wake: leave the idle count before taking a flag
-        if (lane == 0) {
-          const unsigned long long before =
-              atomicAdd(&a.ctl->idle, (1ULL << 32) - 1ULL);  // wakes + 1, idle - 1
-          asm volatile("" ::"l"(before));
-          fence_acq_rel_gpu();
-        }
-        idle = false;
-        __syncwarp();
-      }
-      while (mask) {
+      if (!mask) continue;
+      // wake: leave the idle count (before any word is taken down, below)
+      bool woke = idle;
+      if (idle && lane == 0) atomicAdd(&a.ctl->idle, (1ULL << 32) - 1ULL);
+      idle = false;
+      fence_acq_rel_gpu();  // acquire: the writes published before the flags
+      while (mask && taken < kTakeTiles) {
         const int l = __ffs(mask) - 1;
         mask &= mask - 1;
         const int tile = base + l * W;
-        int got = 0;
-        if (lane == 0) {
-          // ordered: clear the priority before taking the flag, so a value
-          // published in between keeps a priority (at worst a stale one)
-          if (ordered_sched(SCHED)) atomicExch(&a.prio[tile], kClean);
-          got = atomicExch(&a.dirty[tile], 0);
-          if (got) {
-            unflushed++;
-            fence_acq_rel_gpu();  // acquire: the writes published before the flag
-          }
+        if (taken) {  // earlier visits took time: what is pending now
+          if (lane == l) f = *(volatile int *)&a.dirty[tile];
+          fence_acq_rel_gpu();
         }
-        got = __shfl_sync(0xffffffffu, got, 0);
-        if (!got) continue;
-        did = true;
-        relax_tile<KIND, SCHED>(a, t, lane, tile, got);
-        if (++taken == kTakeTiles) break;
+        const int got = __shfl_sync(0xffffffffu, f, l);
+        // ordered: clear the priority first, so a value published during the
+        // visit keeps one (at worst a stale one)
+        if (ordered_sched(SCHED) && lane == 0) atomicExch(&a.prio[tile], kClean);
+        unflushed++;
+        taken++;
+        const bool fenced = relax_tile<KIND, SCHED>(a, t, lane, tile, got);
+        if (woke && !fenced) fence_acq_rel_gpu();
+        woke = false;
+        __syncwarp();
+        if (lane == l) atomicSub(&a.dirty[tile], got);  // the lane that polls this word
       }
-      if (taken == kTakeTiles) break;
     }
     int wait_min = kClean;
     if (ordered_sched(SCHED)) {  // report this warp's waiting work
@@ -527,7 +549,7 @@ relax_persistent_kernel(RelaxArgs a) {
       if (lane == 0 && wait_min != posted) *(volatile int *)&a.wmin[wid] = wait_min;
       posted = wait_min;
     }
-    if (did) {
+    if (taken) {
       spins = 0;
       continue;
     }
@@ -535,33 +557,31 @@ relax_persistent_kernel(RelaxArgs a) {
       idle = true;
       fence_acq_rel_gpu();  // every lane: its flags (and wait report) before the idle mark
       __syncwarp();
-      unsigned long long seen = 0;
-      if (lane == 0) {
-        seen = atomicAdd(&a.ctl->idle, 1ULL) + 1ULL;
-        if ((unsigned)seen == (unsigned)W) fence_acq_rel_gpu();  // all flags visible
-      }
-      seen = __shfl_sync(0xffffffffu, seen, 0);
-      if ((unsigned)seen == (unsigned)W) {
-        if (!ordered_sched(SCHED) || !raise_threshold<SCHED>(a, lane, W, thr))
-          check_done(a, lane, T, seen);
-        raised_at = thr;
-      }
+      if (lane == 0) atomicAdd(&a.ctl->idle, 1ULL);
       continue;
     }
-    if (ordered_sched(SCHED) && wait_min != kClean && raised_at != thr &&
-        (unsigned)*(volatile unsigned long long *)&a.ctl->idle == (unsigned)W) {
-      // every warp idle and this one still waiting: open the next band
-      raise_threshold<SCHED>(a, lane, W, thr);
-      raised_at = thr;
+    if ((unsigned)idle_word == (unsigned)W) {  // every warp was idle at this poll
+      if (ordered_sched(SCHED) && (wid == 0 || (wait_min != kClean && raised_at != thr))) {
+        // open the next band; without one, the run may be over
+        fence_acq_rel_gpu();
+        raised_at = thr;
+        if (!raise_threshold<SCHED>(a, lane, W, thr) && wid == 0)
+          check_done(a, lane, T, idle_word);
+      } else if (!ordered_sched(SCHED) && wid == 0) {
+        check_done(a, lane, T, idle_word);
+      }
     }
     int stop = 0;
     if (lane == 0) {
       if (++spins > kSpinLimit) {
         atomicOr(&a.ctl->abort, ABORT_SPIN);
         stop = 1;
-      } else {
-        // a warp that owns one tile waits on one flag: it polls at once
-        if (T > W || spins > 256) __nanosleep(spins < 64 ? 64 : 512);
+      } else if ((T > W && wid != 0) || spins > 4096) {
+        // a warp that owns one tile waits on one flag, and warp 0 ends the
+        // run: they poll at once.  The others' polls take issue slots and L2
+        // accesses from the warps at work (64 to 512 ns between them instead:
+        // 4096^2 1.04 / 2.27 against 1.01 / 2.23 ms).
+        __nanosleep(1000);
       }
     }
     if (__shfl_sync(0xffffffffu, stop, 0)) break;
@@ -570,8 +590,9 @@ relax_persistent_kernel(RelaxArgs a) {
 }
 
 // Relaxes one tile to its local fixpoint and marks changed neighbours dirty.
+// Returns whether it passed a device-wide fence after its stores.
 template <int KIND, int SCHED>
-__device__ void relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, int mode) {
+__device__ bool relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, int mode) {
   const int ti = tile % a.tm, tj = tile / a.tm;
   const int64_t i0 = (int64_t)ti * kTile, j0 = (int64_t)tj * kTile;
 
@@ -651,7 +672,7 @@ __device__ void relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
 
   // Marks in the column layout: lane l holds interior column l + 1, bit k =
   // interior row k + 1.  An edge visit starts from the ring next to the halo.
-  uint32_t nd = ((mode & DIRTY_FULL) || lane == 0 || lane == kTile - 1) ? 0xffffffffu
+  uint32_t nd = (mode >= DIRTY_FULL || lane == 0 || lane == kTile - 1) ? 0xffffffffu
                                                                        : 0x80000001u;
   uint32_t dm = 0, dmr = 0;  // changed pixels, column and row layout
 
@@ -659,54 +680,18 @@ __device__ void relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
   // Down and up run in the column layout, right and left in the row layout
   // (the marks are transposed between the two).
   constexpr int kCap = (!ordered_sched(SCHED) && (SCHED & 2)) ? kCapSweeps : kMaxSweeps;
-  bool done = false;
+  bool rows = !ordered_sched(SCHED) && (SCHED & 1);
+  // The longest chain of visits takes 6 to 12 sweeps in each tile, many more
+  // than a value needs to cross one.  So the fill publishes its edges after
+  // each pair of sweeps and goes on (fill 512^2 161 -> 139 us, 4096^2 1.36 ->
+  // 1.16 ms, 16384^2 6.73 -> 6.31 ms); gwdt, whose tiles then run more often
+  // on distances that fall again, only at the end (4096^2 2.30 against 2.58 ms).
+  constexpr bool kEager = KIND == FILL;
+  bool fenced = false;
   int sweeps = 0;
-  auto rows = [&]() {  // right and left in the row layout
-    uint32_t ndr = transpose32(nd, lane);
-    sweep<KIND, true, +1>(t, lane, ndr, dmr);
-    sweeps++;
-    if (__any_sync(0xffffffffu, ndr != 0)) {
-      sweep<KIND, true, -1>(t, lane, ndr, dmr);
-      sweeps++;
-    }
-    nd = transpose32(ndr, lane);
-  };
-  while (sweeps < kCap) {
-    if (!__any_sync(0xffffffffu, nd != 0)) {
-      done = true;
-      break;
-    }
-    if (!ordered_sched(SCHED) && (SCHED & 1)) {
-      rows();
-      if (!__any_sync(0xffffffffu, nd != 0)) {
-        done = true;
-        break;
-      }
-    }
-    sweep<KIND, false, +1>(t, lane, nd, dm);
-    sweeps++;
-    if (!__any_sync(0xffffffffu, nd != 0)) {
-      done = true;
-      break;
-    }
-    sweep<KIND, false, -1>(t, lane, nd, dm);
-    sweeps++;
-    if (ordered_sched(SCHED) || !(SCHED & 1)) {
-      if (!__any_sync(0xffffffffu, nd != 0)) {
-        done = true;
-        break;
-      }
-      rows();
-    }
-  }
-
-  // Write back changed cells, coalesced per column: lane = row, bit c of
-  // `dmr` = column c.  (Off-grid cells never change.)
-  dmr |= transpose32(dm, lane);
-  const uint32_t cols = __reduce_or_sync(0xffffffffu, dmr);
-  if (!cols && done) return;
-  {
-    float *const out = a.state + (j0 * a.m + i0 + lane);
+  float *const out = a.state + (j0 * a.m + i0 + lane);  // column 0, row `lane`
+  auto write_columns = [&]() {  // every changed cell, coalesced per column
+    const uint32_t cols = __reduce_or_sync(0xffffffffu, dmr);
 #pragma unroll 1
     for (int c0 = 0; c0 < kTile; c0 += 8) {
       if (!((cols >> c0) & 0xffu)) continue;
@@ -714,70 +699,119 @@ __device__ void relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
       for (int u = 0; u < 8; u++)
         if ((dmr >> (c0 + u)) & 1u) out[(c0 + u) * a.m] = t.s[c0 + u + 1][lane + 1];
     }
-  }
-  // A neighbour needs a visit only if a value of this tile lowers a pixel of
-  // it: the halo holds its values as they were staged, and they only fall,
-  // so a pixel that is not lowered here cannot be lowered there either.
-  // (Four to five in ten visits found nothing to lower without this test:
-  // 16384^2 fill 7.4 -> 6.9 ms, gwdt 11.9 -> 10.4 ms.)
-  constexpr auto at = WarpTile::s_at;
-  const uint32_t row0 = __shfl_sync(0xffffffffu, dmr, 0);
-  const uint32_t row31 = __shfl_sync(0xffffffffu, dmr, kTile - 1);
-  const uint32_t left = __ballot_sync(0xffffffffu, dmr & 1u);
-  const uint32_t right = __ballot_sync(0xffffffffu, dmr >> 31);
-  const bool to_top = row0 && __any_sync(0xffffffffu, lowers<KIND>(t, at(lane + 1, 0), at(lane + 1, 1), kPitch));
-  const bool to_bottom =
-      row31 && __any_sync(0xffffffffu, lowers<KIND>(t, at(lane + 1, kTile + 1), at(lane + 1, kTile), kPitch));
-  const bool to_left = left && __any_sync(0xffffffffu, lowers<KIND>(t, at(0, lane + 1), at(1, lane + 1), 1));
-  const bool to_right =
-      right && __any_sync(0xffffffffu, lowers<KIND>(t, at(kTile + 1, lane + 1), at(kTile, lane + 1), 1));
-
-  // Lanes 0..8 mark one neighbour each with an atomic OR, after a release
-  // fence.  A tile whose edges did not change publishes nothing: only its
-  // owner reads its interior again.
-  int tgt = -1, val = DIRTY_EDGE;
-  switch (lane) {
-    case 0: if (to_top) { tgt = 0; } break;
-    case 1: if (to_bottom) { tgt = 1; } break;
-    case 2: if (to_left) { tgt = 2; } break;
-    case 3: if (to_right) { tgt = 3; } break;
-    case 4: case 5: case 6: case 7: {  // corners: column 0 / 31, row 0 / 31
-      const int c = lane < 6 ? 0 : kTile + 1, r = (lane & 1) ? kTile + 1 : 0;
-      const int cn = lane < 6 ? 1 : kTile, rn = (lane & 1) ? kTile : 1;
-      const uint32_t edge = lane < 6 ? left : right;
-      if (((edge >> (rn - 1)) & 1u) && lowers<KIND>(t, at(c, r), at(cn, rn), 0)) tgt = lane;
-      break;
+  };
+  for (;;) {
+    if (!rows) {
+      sweep<KIND, false, +1>(t, lane, nd, dm);
+      sweeps++;
+      if (__any_sync(0xffffffffu, nd != 0)) {
+        sweep<KIND, false, -1>(t, lane, nd, dm);
+        sweeps++;
+      }
+    } else {
+      uint32_t ndr = transpose32(nd, lane);
+      sweep<KIND, true, +1>(t, lane, ndr, dmr);
+      sweeps++;
+      if (__any_sync(0xffffffffu, ndr != 0)) {
+        sweep<KIND, true, -1>(t, lane, ndr, dmr);
+        sweeps++;
+      }
+      nd = transpose32(ndr, lane);
     }
-    case 8: if (!done) { tgt = 8; val = DIRTY_FULL; } break;  // capped: revisit
-    default: break;
+    rows = !rows;
+    const bool done = !__any_sync(0xffffffffu, nd != 0);
+    if (!done && !kEager && sweeps < kCap) continue;
+
+    // Publish.  Changed cells so far, lane = row, bit c of `dmr` = column c
+    // (off-grid cells never change).  The edges are what neighbours wait
+    // for: they are written and published first, the interior at the end.
+    if (done && !__any_sync(0xffffffffu, (dm | dmr) != 0)) return fenced;  // nothing changed
+    dmr |= transpose32(dm, lane);
+    dm = 0;
+    const uint32_t row0 = __shfl_sync(0xffffffffu, dmr, 0);
+    const uint32_t row31 = __shfl_sync(0xffffffffu, dmr, kTile - 1);
+    const uint32_t left = __ballot_sync(0xffffffffu, dmr & 1u);
+    const uint32_t right = __ballot_sync(0xffffffffu, dmr >> 31);
+    if (kEager) {
+      if ((row0 >> lane) & 1u) a.state[(j0 + lane) * a.m + i0] = t.s[lane + 1][1];
+      if ((row31 >> lane) & 1u) a.state[(j0 + lane) * a.m + i0 + kTile - 1] = t.s[lane + 1][kTile];
+      if (dmr & 1u) out[0] = t.s[1][lane + 1];
+      if (dmr >> 31) out[(kTile - 1) * a.m] = t.s[kTile][lane + 1];
+    } else {
+      write_columns();
+    }
+    // A neighbour needs a visit only if a value of this tile lowers a pixel
+    // of it: the halo holds its values as they were staged, and they only
+    // fall, so a pixel that is not lowered here cannot be lowered there
+    // either.  (Four to five in ten visits found nothing to lower without
+    // this test: 16384^2 fill 7.4 -> 6.9 ms, gwdt 11.9 -> 10.4 ms.)
+    constexpr auto at = WarpTile::s_at;
+    const bool to_top =
+        row0 && __any_sync(0xffffffffu, lower<KIND>(t, at(lane + 1, 0), at(lane + 1, 1), kPitch));
+    const bool to_bottom =
+        row31 && __any_sync(0xffffffffu, lower<KIND>(t, at(lane + 1, kTile + 1),
+                                                     at(lane + 1, kTile), kPitch));
+    const bool to_left =
+        left && __any_sync(0xffffffffu, lower<KIND>(t, at(0, lane + 1), at(1, lane + 1), 1));
+    const bool to_right =
+        right && __any_sync(0xffffffffu, lower<KIND>(t, at(kTile + 1, lane + 1),
+                                                     at(kTile, lane + 1), 1));
+    // Lanes 0..8 add to one neighbour's word each, after a release fence.  A
+    // tile that lowers no neighbour publishes nothing: only its owner reads
+    // its interior again.
+    int tgt = -1, val = DIRTY_EDGE;
+    switch (lane) {
+      case 0: if (to_top) { tgt = 0; } break;
+      case 1: if (to_bottom) { tgt = 1; } break;
+      case 2: if (to_left) { tgt = 2; } break;
+      case 3: if (to_right) { tgt = 3; } break;
+      case 4: case 5: case 6: case 7: {  // corners: column 0 / 31, row 0 / 31
+        const int c = lane < 6 ? 0 : kTile + 1, r = (lane & 1) ? kTile + 1 : 0;
+        const int cn = lane < 6 ? 1 : kTile, rn = (lane & 1) ? kTile : 1;
+        const uint32_t edge = lane < 6 ? left : right;
+        if (((edge >> (rn - 1)) & 1u) && lower<KIND>(t, at(c, r), at(cn, rn), 0)) tgt = lane;
+        break;
+      }
+      case 8:  // capped: revisit
+        if (!done && sweeps >= kCap) { tgt = 8; val = DIRTY_FULL; }
+        break;
+      default: break;
+    }
+    if (tgt >= 0) {
+      const int di = (tgt == 0 || tgt == 4 || tgt == 6) ? -1 : (tgt == 1 || tgt == 5 || tgt == 7) ? 1 : 0;
+      const int dj = (tgt == 2 || tgt == 4 || tgt == 5) ? -1 : (tgt == 3 || tgt == 6 || tgt == 7) ? 1 : 0;
+      const int ni = ti + di, nj = tj + dj;
+      tgt = (ni < 0 || nj < 0 || ni >= a.tm || nj >= a.tn) ? -1 : nj * a.tm + ni;
+    }
+    // Every lane fences its own stores, then the warp barrier orders those
+    // fences before the atomics (the fence-then-barrier publication
+    // pattern): a warp that reads a word and fences sees every store made
+    // before it.
+    if (__any_sync(0xffffffffu, tgt >= 0)) {
+      int key = kUrgent;
+      if (ordered_sched(SCHED)) {  // the lowest changed value on the tile's edges
+        float v = INFINITY;
+        if ((row0 >> lane) & 1u) v = fminf(v, t.s[lane + 1][1]);
+        if ((row31 >> lane) & 1u) v = fminf(v, t.s[lane + 1][kTile]);
+        if ((left >> lane) & 1u) v = fminf(v, t.s[1][lane + 1]);
+        if ((right >> lane) & 1u) v = fminf(v, t.s[kTile][lane + 1]);
+        key = __reduce_min_sync(0xffffffffu, value_key(v));
+        if (tgt >= 0 && val == DIRTY_FULL) key = kUrgent;  // a capped visit resumes at once
+      }
+      fence_acq_rel_gpu();
+      __syncwarp();
+      fenced = true;
+      if (tgt >= 0) {
+        if (ordered_sched(SCHED)) atomicMin(&a.prio[tgt], key);
+        atomicAdd(&a.dirty[tgt], val);
+      }
+    }
+    if (done || sweeps >= kCap) break;
+    __syncwarp();  // the halo as lowered, before the next sweep
   }
-  if (tgt >= 0) {
-    const int di = (tgt == 0 || tgt == 4 || tgt == 6) ? -1 : (tgt == 1 || tgt == 5 || tgt == 7) ? 1 : 0;
-    const int dj = (tgt == 2 || tgt == 4 || tgt == 5) ? -1 : (tgt == 3 || tgt == 6 || tgt == 7) ? 1 : 0;
-    const int ni = ti + di, nj = tj + dj;
-    tgt = (ni < 0 || nj < 0 || ni >= a.tm || nj >= a.tn) ? -1 : nj * a.tm + ni;
-  }
-  // Every lane fences its own stores, then the warp barrier orders those
-  // fences before the flag atomics (the fence-then-barrier publication
-  // pattern): a warp that takes a flag and fences sees every store made
-  // before it.
-  if (!__any_sync(0xffffffffu, tgt >= 0)) return;
-  int key = kUrgent;
-  if (ordered_sched(SCHED)) {  // the lowest changed value on the tile's edges
-    float v = INFINITY;
-    if ((row0 >> lane) & 1u) v = fminf(v, t.s[lane + 1][1]);
-    if ((row31 >> lane) & 1u) v = fminf(v, t.s[lane + 1][kTile]);
-    if ((left >> lane) & 1u) v = fminf(v, t.s[1][lane + 1]);
-    if ((right >> lane) & 1u) v = fminf(v, t.s[kTile][lane + 1]);
-    key = __reduce_min_sync(0xffffffffu, value_key(v));
-    if (tgt >= 0 && val == DIRTY_FULL) key = kUrgent;  // a capped visit resumes at once
-  }
-  fence_acq_rel_gpu();
-  __syncwarp();
-  if (tgt >= 0) {
-    if (ordered_sched(SCHED)) atomicMin(&a.prio[tgt], key);
-    atomicOr(&a.dirty[tgt], val);
-  }
+
+  if (kEager) write_columns();
+  return fenced;
 }
 
 // f = dem where bc == 1 (and where dem is NaN), +INF elsewhere

@@ -125,7 +125,9 @@ class Workspace {
 // kRecordInts ints: {kind, a, b, c}.
 constexpr int kRecordInts = 4;
 enum : int { REC_RELAX = 1, REC_FOREST = 2 };
-constexpr int kRelaxAbort = 5;  // int of a relaxation's control block: its abort word
+// Ints of a relaxation's control block: its abort word, its visits (two ints).
+constexpr int kRelaxAbort = 3;
+constexpr int kRelaxVisits = 4;
 struct StatusSink {
   int *dev;      // device array of records
   int capacity;  // records
@@ -242,9 +244,9 @@ tt_cuda_status identifyflats_dev(int32_t *flags, const float *dem,
                                  const GridDims &g,
                                  unsigned long long *count_dev,
                                  cudaStream_t st);
-// Tile flags of the relaxations: a tile waits with its edge ring or its
-// whole interior to be evaluated.
-enum : int { DIRTY_EDGE = 1, DIRTY_FULL = 2 };
+// Tile flags of the relaxations: a tile waits with its edge ring (any number
+// of DIRTY_EDGE) or its whole interior (DIRTY_FULL or more) to be evaluated.
+enum : int { DIRTY_EDGE = 1, DIRTY_FULL = 1 << 20 };
 // Marks dirty (whole interior) the tiles whose pixels or halo hold pixel
 // (i, j) of an m x n grid with tm tiles along i.
 __device__ __forceinline__ void mark_tiles_near(int *dirty, int tm, int64_t i, int64_t j,

@@ -203,7 +203,7 @@ tt_cuda_status CallArena::collect(int tiles, cudaStream_t st) {
     if (r != TT_CUDA_SUCCESS) s = r;
     if (kind_[k] == REC_RELAX && !sink) {
       unsigned long long visits;
-      std::memcpy(&visits, b, 8);
+      std::memcpy(&visits, b + kRelaxVisits, 8);
       set_last_rounds((int64_t)(visits / (unsigned long long)(tiles > 0 ? tiles : 1)));
     }
   }
