@@ -24,14 +24,24 @@
 //
 // GPU form.  The edges are grouped by target and by source (radix sort of
 // (node, edge) keys), so each node's in- and out-edges are in list order.
-// pend(e) counts the in-edges of u listed before e.  Walks start at edges
-// with pend 0; a walker computes val(e) by pulling the values of those
-// in-edges in list order, then counts itself off every out-edge of v listed
-// after e, and continues with each edge whose count it took to zero (a
-// small private stack, spilling to a global work list that a further launch
-// drains).  Every edge is computed exactly once, by the last contributor to
-// arrive, and every sum is taken in list order in FP64: the result does not
-// depend on thread timing and is rounded once to float32.
+// need(e) counts the in-edges of u listed before e.  Walks start at edges
+// with need 0; a walker computes val(e) from the values of those in-edges in
+// list order, then announces it to every out-edge of v listed after e, and
+// continues with each edge whose last value it brought (a small private
+// stack, spilling to a global work list that a further launch drains).
+// Every edge is computed exactly once, by the last contributor to arrive,
+// and every sum is taken in list order in FP64: the result does not depend
+// on thread timing and is rounded once to float32.
+//
+// The longest chain of edges bounds the sweep: a river of thousands of
+// pixels, one edge after the other.  So a hop reads one 32-byte record,
+// fetched while the hop before is under way, and waits for as little as the
+// next edge allows: for nothing when this value is the only one it needs,
+// for one exchange of values when it needs two (the second to arrive gets
+// the first's value back and leaves with both), and for a count and the
+// values, read at the same time, when it needs more.  2001 x 3003 forest with
+// fractions: walks of 2.1 ms (14.4 ms with a count, two fences and about
+// eight dependent accesses a hop).
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
@@ -44,7 +54,19 @@ namespace {
 
 constexpr int kWalkStack = 24;
 
-enum : int { EF_BAD_INDEX = 1, EF_CYCLE = 2 };
+enum : int { EF_BAD_INDEX = 1, EF_WAIT = 2 };
+
+// What a walker needs of an edge e = (u, v), in one sector.
+struct __align__(32) EdgeRec {
+  int in_lo;   // first value slot of the in-edges of u
+  int need;    // in-edges of u listed before e
+  int slot;    // value slot of e: its place among the edges by target
+  unsigned w;  // start value of u, the output type's bits
+  unsigned f;  // factor of e, its type's bits
+  int out_lo;  // the out-edges of v listed after e: out_list[out_lo, out_hi)
+  int out_hi;
+  int next;    // the first of them, -1 without one
+};
 
 struct FlowArgs {
   const ptrdiff_t *src;
@@ -57,11 +79,16 @@ struct FlowArgs {
   const int *in_list;  // ... in list order
   const int *out_off;  // N + 1: edges out of each node ...
   const int *out_list;
-  int *pend;      // per edge: earlier in-edges of its source not yet computed
-  void *val;      // per edge, 8 bytes: double (+, *) or uint32 (|, &)
+  EdgeRec *rec;   // per edge
+  int *pend;      // per edge that needs three values or more: those missing
+  unsigned long long *meet;  // per edge that needs two: the first to arrive (kEmpty: none)
+  unsigned long long *val;   // per value slot: the value's bits (kEmpty: none yet)
   int *work;      // spill list of ready edges (each edge enters at most once)
   int *ctl;       // [0] spill count, [1] edges computed, [2] error bits
 };
+
+// No value: a NaN whose low bits no float's NaN has, and no 32-bit word.
+constexpr unsigned long long kEmpty = ~0ULL;
 
 // Edge e of the swept list: its source, target and list position.
 __device__ __forceinline__ int64_t e_src(const FlowArgs &a, int64_t e) {
@@ -77,30 +104,34 @@ __device__ __forceinline__ int64_t e_pos(const FlowArgs &a, int64_t e) {
 // The two semirings.
 struct AddMul {  // (+, *) carried in FP64, float in and out
   using T = double;
-  static __device__ T start(const FlowArgs &a, int64_t u) {
-    return a.w ? (double)static_cast<const float *>(a.w)[u] : 1.0;
+  static __device__ unsigned one() { return 0x3f800000u; }  // 1.0f
+  static __device__ T start(unsigned w) { return (double)__uint_as_float(w); }
+  static __device__ T add(T s, T x) { return __dadd_rn(s, x); }
+  static __device__ T mul(unsigned f, T s) { return __dmul_rn((double)__uint_as_float(f), s); }
+  static __device__ unsigned long long bits(T x) {
+    return (unsigned long long)__double_as_longlong(x);
   }
-  static __device__ T add(T s, T x) { return s + x; }
-  static __device__ T mul(const FlowArgs &a, int64_t e, T s) {
-    return (double)static_cast<const float *>(a.frac)[e_pos(a, e)] * s;
-  }
+  static __device__ T value(unsigned long long b) { return __longlong_as_double((long long)b); }
   static __device__ void store(void *out, int64_t v, T s) {
     static_cast<float *>(out)[v] = (float)s;
   }
 };
 struct OrAnd {  // (|, &) on 32-bit words, exact
   using T = uint32_t;
-  static __device__ T start(const FlowArgs &a, int64_t u) {
-    return a.w ? static_cast<const uint32_t *>(a.w)[u] : 0xffffffffu;
-  }
+  static __device__ unsigned one() { return 0xffffffffu; }
+  static __device__ T start(unsigned w) { return w; }
   static __device__ T add(T s, T x) { return s | x; }
-  static __device__ T mul(const FlowArgs &a, int64_t e, T s) {
-    return static_cast<const uint32_t *>(a.frac)[e_pos(a, e)] & s;
-  }
+  static __device__ T mul(unsigned f, T s) { return f & s; }
+  static __device__ unsigned long long bits(T x) { return x; }
+  static __device__ T value(unsigned long long b) { return (T)b; }
   static __device__ void store(void *out, int64_t v, T s) {
     static_cast<uint32_t *>(out)[v] = s;
   }
 };
+template <class S>
+__device__ __forceinline__ unsigned start_bits(const FlowArgs &a, int64_t u) {
+  return a.w ? static_cast<const unsigned *>(a.w)[u] : S::one();
+}
 
 int list_grid(int64_t n) {
   int64_t b = (n + 255) / 256;
@@ -149,32 +180,102 @@ __device__ __forceinline__ int first_after(const int *list, int lo, int hi, int 
   return lo;
 }
 
-// pend(e) = in-edges of src(e) listed before e; edges with none start walks.
-__global__ void ef_pend_kernel(FlowArgs a, int *__restrict__ starts, int *__restrict__ nstart) {
+// Value slot of every edge: its place among the edges sorted by target.
+__global__ void ef_slot_kernel(FlowArgs a, int *__restrict__ slot) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.E;
+       i += (int64_t)gridDim.x * blockDim.x)
+    slot[a.in_list[i]] = (int)i;
+}
+
+// The edges' records; edges that need no value start walks.
+template <class S>
+__global__ void ef_record_kernel(FlowArgs a, const int *__restrict__ slot,
+                                 int *__restrict__ starts, int *__restrict__ nstart) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < a.E;
        e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t u = e_src(a, e);
-    const int lo = a.in_off[u];
-    const int p = first_after(a.in_list, lo, a.in_off[u + 1], (int)e - 1) - lo;
-    a.pend[e] = p;
-    if (p == 0) starts[append_slot(nstart)] = (int)e;
+    const int64_t u = e_src(a, e), v = e_tgt(a, e);
+    EdgeRec r;
+    r.in_lo = a.in_off[u];
+    r.need = first_after(a.in_list, r.in_lo, a.in_off[u + 1], (int)e - 1) - r.in_lo;
+    r.slot = slot[e];
+    r.w = start_bits<S>(a, u);
+    r.f = static_cast<const unsigned *>(a.frac)[e_pos(a, e)];
+    r.out_hi = a.out_off[v + 1];
+    r.out_lo = first_after(a.out_list, a.out_off[v], r.out_hi, (int)e);
+    r.next = r.out_lo < r.out_hi ? a.out_list[r.out_lo] : -1;
+    a.rec[e] = r;
+    a.pend[e] = r.need;
+    a.meet[e] = kEmpty;
+    a.val[e] = kEmpty;
+    if (r.need == 0) starts[append_slot(nstart)] = (int)e;
   }
 }
 
-// Value of node u just before edge x is applied: w(u) plus the values of
-// its in-edges listed before x, in list order.
+__device__ __forceinline__ EdgeRec load_record(const EdgeRec *rec, int e) {
+  const int4 *p = reinterpret_cast<const int4 *>(rec + e);
+  const int4 a = __ldg(p), b = __ldg(p + 1);
+  return EdgeRec{a.x, a.y, a.z, (unsigned)a.w, (unsigned)b.x, b.y, b.z, b.w};
+}
+
+// Start value of the edge's source plus the values of the in-edges the edge
+// needs, in list order, from memory.  Every one of them has been stored; one
+// that is not visible yet is read again (kWaitReads bounds that, far above
+// the time a store takes).
+constexpr int kWaitReads = 1 << 20;
+constexpr int kReadAhead = 8;
+
+__device__ __forceinline__ unsigned long long read_value(const unsigned long long *p) {
+  return *(const volatile unsigned long long *)p;
+}
+
 template <class S>
-__device__ __forceinline__ typename S::T value_before(const FlowArgs &a, int64_t u, int x) {
-  using T = typename S::T;
-  T s = S::start(a, u);
-  const T *val = static_cast<const T *>(a.val);
-  const int hi = a.in_off[u + 1];
-  for (int k = a.in_off[u]; k < hi; k++) {
-    const int e2 = a.in_list[k];
-    if (e2 >= x) break;
-    s = S::add(s, __ldcg(&val[e2]));
+__device__ __forceinline__ typename S::T sum_needed(const FlowArgs &a, const EdgeRec &r,
+                                                    const unsigned long long *ahead, int n) {
+  typename S::T s = S::start(r.w);
+  const unsigned long long *val = a.val + r.in_lo;
+  for (int k = 0; k < r.need; k++) {
+    unsigned long long b = kEmpty;
+#pragma unroll
+    for (int q = 0; q < kReadAhead; q++)
+      if (q == k && q < n) b = ahead[q];
+    for (int it = 0; b == kEmpty; it++) {
+      if (it == kWaitReads) {
+        atomicOr(&a.ctl[2], EF_WAIT);
+        break;
+      }
+      b = read_value(&val[k]);
+    }
+    s = S::add(s, S::value(b));
   }
   return s;
+}
+
+// Brings the value `x` in value slot `slot` to edge o (record r).  True when
+// it was the last value o needs; s is then the sum o carries on.
+template <class S>
+__device__ __forceinline__ bool arrive(const FlowArgs &a, int o, const EdgeRec &r, int slot,
+                                       typename S::T x, typename S::T &s) {
+  if (r.need == 1) {
+    s = S::add(S::start(r.w), x);
+    return true;
+  }
+  if (r.need == 2) {
+    const unsigned long long first = atomicExch(&a.meet[o], S::bits(x));
+    if (first == kEmpty) return false;
+    const typename S::T y = S::value(first);
+    s = slot == r.in_lo ? S::add(S::add(S::start(r.w), x), y)
+                        : S::add(S::add(S::start(r.w), y), x);
+    return true;
+  }
+  // The values are read while the count is under way: no fence, a value
+  // that is announced but not visible yet reads as kEmpty and is read again.
+  unsigned long long ahead[kReadAhead];
+#pragma unroll
+  for (int k = 0; k < kReadAhead; k++)
+    ahead[k] = k < r.need ? read_value(a.val + r.in_lo + k) : kEmpty;
+  if (atomicSub(&a.pend[o], 1) != 1) return false;
+  s = sum_needed<S>(a, r, ahead, kReadAhead);
+  return true;
 }
 
 // Walks from the ready edges list[base, base + n), n = *n_dev when n_dev is
@@ -182,40 +283,62 @@ __device__ __forceinline__ typename S::T value_before(const FlowArgs &a, int64_t
 template <class S>
 __global__ void ef_walk_kernel(FlowArgs a, const int *__restrict__ list,
                                const int *__restrict__ n_dev, int n_host, int base) {
+  using T = typename S::T;
   const int n = n_dev ? *n_dev : n_host;
   int done = 0;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     int stack[kWalkStack];
+    T sums[kWalkStack];
     int sp = 0;
-    stack[sp++] = list[base + t];
-    while (sp) {
-      const int x = stack[--sp];
-      const int64_t u = e_src(a, x), v = e_tgt(a, x);
-      static_cast<typename S::T *>(a.val)[x] = S::mul(a, x, value_before<S>(a, u, x));
+    // every value the edge needs was stored before this launch
+    EdgeRec r = load_record(a.rec, list[base + t]), rn = {};
+    if (r.next >= 0) rn = load_record(a.rec, r.next);
+    T s = sum_needed<S>(a, r, nullptr, 0);
+    for (;;) {
+      const T x = S::mul(r.f, s);
+      *(volatile unsigned long long *)&a.val[r.slot] = S::bits(x);
       done++;
-      __threadfence();  // val(x) before the counts that announce it
-      const int hi = a.out_off[v + 1];
-      for (int k = first_after(a.out_list, a.out_off[v], hi, x); k < hi; k++) {
-        const int o = a.out_list[k];
-        if (atomicSub(&a.pend[o], 1) != 1) continue;
-        __threadfence();  // every earlier in-edge of v is visible now
-        if (sp < kWalkStack) stack[sp++] = o;
-        else a.work[atomicAdd(&a.ctl[0], 1)] = o;
+      bool on = false;
+      EdgeRec r2 = {};  // of the edge after the next one, read ahead
+      if (r.next >= 0) {
+        if (rn.next >= 0) r2 = load_record(a.rec, rn.next);
+        on = arrive<S>(a, r.next, rn, r.slot, x, s);
+        for (int k = r.out_lo + 1; k < r.out_hi; k++) {  // further out-edges
+          const int o = a.out_list[k];
+          T so;
+          if (!arrive<S>(a, o, load_record(a.rec, o), r.slot, x, so)) continue;
+          if (sp < kWalkStack) {
+            stack[sp] = o;
+            sums[sp++] = so;
+          } else {
+            a.work[atomicAdd(&a.ctl[0], 1)] = o;
+          }
+        }
+      }
+      if (on) {
+        r = rn;
+        rn = r2;
+      } else {
+        if (!sp) break;
+        s = sums[--sp];
+        r = load_record(a.rec, stack[sp]);
+        if (r.next >= 0) rn = load_record(a.rec, r.next);
       }
     }
   }
-  if (done) atomicAdd(&a.ctl[1], done);
+  __syncwarp();
+  done = __reduce_add_sync(0xffffffffu, done);
+  if ((threadIdx.x & 31) == 0 && done) atomicAdd(&a.ctl[1], done);
 }
 
 // out(v) = w(v) + the values of every edge into v, in list order.
 template <class S>
 __global__ void ef_final_kernel(FlowArgs a, void *__restrict__ out) {
   using T = typename S::T;
-  const T *val = static_cast<const T *>(a.val);
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < a.N;
        v += (int64_t)gridDim.x * blockDim.x) {
-    T s = S::start(a, v);
-    for (int k = a.in_off[v]; k < a.in_off[v + 1]; k++) s = S::add(s, val[a.in_list[k]]);
+    T s = S::start(start_bits<S>(a, v));
+    for (int k = a.in_off[v]; k < a.in_off[v + 1]; k++) s = S::add(s, S::value(a.val[k]));
     S::store(out, v, s);
   }
 }
@@ -249,10 +372,11 @@ tt_cuda_status edge_sweep_impl(void *out, const void *w, const ptrdiff_t *source
   const int nbs = scan_blocks_for(N + 1);
   size_t sort_tmp = 0;
   cub::DeviceRadixSort::SortKeys(nullptr, sort_tmp, (unsigned long long *)nullptr,
-                                 (unsigned long long *)nullptr, (int)Em, 0, 64, st);
+                                 (unsigned long long *)nullptr, (int)Em, 32,
+                                 32 + bits_for(N), st);
   Workspace &ws = workspace();
-  const size_t need = 256 + 4 * align_up((size_t)Em * 8) + 2 * align_up((size_t)(N + 1) * 4) +
-                      2 * align_up((size_t)(N + 1) * 4) + 5 * align_up((size_t)Em * 4) +
+  const size_t need = 256 + 6 * align_up((size_t)Em * 8) + 2 * align_up((size_t)(N + 1) * 4) +
+                      2 * align_up((size_t)(N + 1) * 4) + 6 * align_up((size_t)Em * 4) +
                       2 * align_up((size_t)(nbs + 1) * 4) + align_up(sort_tmp) + 4096;
   if (!ws.reserve(need)) return TT_CUDA_ERR_ALLOC;
   int *ctl = (int *)ws.take(256);  // [0] spill, [1] computed, [2] errors, [3] starts
@@ -269,19 +393,22 @@ tt_cuda_status edge_sweep_impl(void *out, const void *w, const ptrdiff_t *source
   int *pend = (int *)ws.take((size_t)Em * 4);
   int *starts = (int *)ws.take((size_t)Em * 4);
   int *work = (int *)ws.take((size_t)Em * 4);
+  int *slot = (int *)ws.take((size_t)Em * 4);
+  unsigned long long *meet = (unsigned long long *)ws.take((size_t)Em * 8);
+  unsigned long long *val = (unsigned long long *)ws.take((size_t)Em * 8);
   int *cnt = (int *)ws.take((size_t)(nbs + 1) * 4);
   int *off = (int *)ws.take((size_t)(nbs + 1) * 4);
   void *tmp = ws.take(sort_tmp);
-  // The values (8 bytes an edge at most) reuse the key buffers, which are
-  // spent once the lists exist.
-  void *val = kin;
+  // The records (32 bytes an edge) reuse the four key buffers, which lie one
+  // after another and are spent once the lists exist.
+  EdgeRec *rec = reinterpret_cast<EdgeRec *>(kin);
 
   TT_CHECK(cudaMemsetAsync(ctl, 0, 256, st));
   TT_CHECK(cudaMemsetAsync(din, 0, (size_t)(N + 1) * 4, st));
   TT_CHECK(cudaMemsetAsync(dout, 0, (size_t)(N + 1) * 4, st));
   const int eg = list_grid(E);
   FlowArgs a{source, target, frac, w, N, E, rev, nullptr, nullptr, nullptr, nullptr,
-             pend, val, work, ctl};
+             rec, pend, meet, val, work, ctl};
   if (E > 0) TT_LAUNCH(ef_keys_kernel, eg, 256, 0, st, a, kin, kout, din, dout, ctl + 2);
   int *h = (int *)pinned_scratch();
   if (!h) return TT_CUDA_ERR_ALLOC;
@@ -295,20 +422,26 @@ tt_cuda_status edge_sweep_impl(void *out, const void *w, const ptrdiff_t *source
   a.out_off = out_off;
   a.out_list = out_list;
   if (E > 0) {
+    // The keys are in edge order and the sort is stable: the nodes' bits are
+    // enough (half the passes: 818 -> 394 us for 6 M edges).
     const int end_bit = 32 + bits_for(N);
     size_t tb = sort_tmp;
-    TT_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kin, sin, (int)E, 0, end_bit, st));
+    TT_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kin, sin, (int)E, 32, end_bit, st));
     tb = sort_tmp;
-    TT_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kout, sout, (int)E, 0, end_bit, st));
+    TT_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kout, sout, (int)E, 32, end_bit, st));
     TT_LAUNCH(ef_extract_kernel, eg, 256, 0, st, sin, sout, E, in_list, out_list);
-    TT_LAUNCH(ef_pend_kernel, eg, 256, 0, st, a, starts, ctl + 3);
-    TT_LAUNCH(ef_walk_kernel<S>, eg, 256, 0, st, a, starts, ctl + 3, 0, 0);
+    TT_LAUNCH(ef_slot_kernel, eg, 256, 0, st, a, slot);
+    TT_LAUNCH(ef_record_kernel<S>, eg, 256, 0, st, a, slot, starts, ctl + 3);
+    // One walker per start (blocks beyond their count exit at once): no start
+    // of a long chain waits for a thread to finish other walks first.
+    TT_LAUNCH(ef_walk_kernel<S>, (int)((E + 255) / 256), 256, 0, st, a, starts, ctl + 3, 0, 0);
     // Drain the spill list: each launch walks the edges spilled by the
     // previous one.  Every edge is spilled at most once, so this ends.
     int base = 0;
     for (int round = 0;; round++) {
-      TT_CHECK(cudaMemcpyAsync(h, ctl, 8, cudaMemcpyDeviceToHost, st));
+      TT_CHECK(cudaMemcpyAsync(h, ctl, 12, cudaMemcpyDeviceToHost, st));
       TT_CHECK(cudaStreamSynchronize(st));
+      if (h[2] & EF_WAIT) return TT_CUDA_ERR_NOT_CONVERGED;
       const int spilled = h[0];
       if (spilled == base) break;
       if (round > E) return TT_CUDA_ERR_CYCLE;  // cannot happen: bounded by E
