@@ -16,7 +16,7 @@
 // maximal depth; the reference picks one of those pixels by its scan-order
 // union-find (src/gwdt.c:141-153), which can differ when depths tie.
 //
-// Work decomposition: one warp per 32 x 32 tile labels the tile's internal
+// Work decomposition: one block per 32 x 32 tile labels the tile's internal
 // edges in shared memory (with path halving) and reduces each tile-local
 // component to its maximum depth and the smallest pixel attaining it; only
 // edges that cross tile borders touch the global union-find, and the global
@@ -68,9 +68,12 @@ __device__ void uf_union(int *L, int a, int b) {
   }
 }
 
-constexpr int kCclWarps = 4;
+constexpr int kCclThreads = 128;
+constexpr int kSlots = kTile * kTile / 2;          // run slots of a tile (see CclTile)
+constexpr int kSlotsPer = kSlots / kCclThreads;    // 4 a thread
+constexpr int kMaxRoots = (kTile / 2) * (kTile / 2);  // 8-connected components of a tile
 
-// Shared-memory union-find over run ids (see ccl_tile_kernel).
+// Shared-memory union-find over run slots (see ccl_tile_kernel).
 __device__ __forceinline__ int sfind(int *lab, int x) {
   volatile int *v = lab;
   int p = v[x];
@@ -120,214 +123,187 @@ __device__ __forceinline__ unsigned long long pack_best(int key, int loc) {
   return ((unsigned long long)((unsigned)key ^ 0x80000000u) << 32) | (unsigned)(1023 - loc);
 }
 
+// Two run starts of a column are at least two rows apart, so column * 16 +
+// (first row) / 2 numbers the runs of a tile: 512 slots.
 struct CclTile {
-  // Union-find over run ids (column * 32 + first row).  Two run starts of
-  // one column are at least two rows apart, so start >> 1 gives every run
-  // its own 64-bit slot: once every run knows its root, lab64 holds the
-  // per-root reduction (pack_best), and each run parks its own best in
-  // key64 at its start (its pixels' keys are read by then).
-  union {
-    int lab[kTile * kTile];
-    unsigned long long lab64[kTile * kTile / 2];
-  };
-  union {
-    int key[kTile * kTile];  // per pixel: depth key (INT_MIN: none)
-    unsigned long long key64[kTile * kTile / 2];
-  };
-  int16_t root[kTile * kTile];  // per pixel: local root, -1 for non-flats
-  uint32_t starts[kTile];       // run starts of each column
+  uint32_t mask[kTile];               // flat mask of each column (bit = row)
+  int lab[kSlots];                    // union-find over run slots
+  int key[kTile * kTile];             // per pixel: depth key (INT_MIN: none)
+  unsigned long long best[kSlots];    // per root slot: the component's pack_best
+  int warp_roots[kCclThreads / 32];
+  int base;
 };
 
-// One warp per tile.  Each lane owns one column's flat mask (32 bits): a
-// vertical run of flats is connected by construction, so the union-find only
-// runs over runs, uniting each run with the runs of the next column that
-// touch it (8-connectivity = its extent grown by one row).  Every pixel then
-// takes the root of its run; each tile-local component is reduced to its
-// maximum depth and the smallest pixel attaining it.
-__global__ void __launch_bounds__(kCclWarps * 32)
-ccl_tile_kernel(int *__restrict__ L, int *__restrict__ lmax, int *__restrict__ larg,
-                unsigned long long *__restrict__ best,
-                int *__restrict__ roots, int *__restrict__ nroots,
-                uint4 *__restrict__ edges,
-                const int32_t *__restrict__ flats, const float *__restrict__ orig,
-                const float *__restrict__ filled, int64_t m, int64_t n, int tm, int tn) {
-  __shared__ CclTile tiles[kCclWarps];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  CclTile &t = tiles[warp];
-  const int T = tm * tn;
-  for (int tile = blockIdx.x * kCclWarps + warp; tile < T; tile += gridDim.x * kCclWarps) {
-    const int ti = tile % tm, tj = tile / tm;
-    const int64_t i0 = (int64_t)ti * kTile, j0 = (int64_t)tj * kTile;
-    const int64_t i = i0 + lane;  // lane = row for the per-pixel phases
-    uint32_t my_mask = 0;
-    // Eight columns at a time: every load of the batch is issued (from a
-    // clamped, always valid address) before any result is used.
+// A tile-local component: its root pixel (the first pixel of its first run),
+// its largest depth key and the smallest pixel attaining it (INT_MAX: none).
+struct __align__(16) LocalRoot {
+  int pixel, key, arg, pad;
+};
+
+__device__ __forceinline__ uint32_t run_starts(uint32_t m) { return m & ~(m << 1); }
+// First row of the run in slot k of a column with run starts s, -1 without one.
+__device__ __forceinline__ int slot_row(uint32_t s, int k) {
+  const uint32_t two = (s >> (2 * k)) & 3u;
+  return two ? 2 * k + (int)(two >> 1) : -1;
+}
+
+// One block of four warps per tile.  A vertical run of flats is connected by
+// construction, so the union-find only runs over runs, uniting each run with
+// the runs of the column before that touch it (8-connectivity = its extent
+// grown by one row).  Threads take run slots, four each, so that the serial
+// parts -- unions, and a run's best pixel -- are at most four runs a thread;
+// a warp per tile with a lane per column stepped through up to sixteen, half
+// of its lanes idle (14.7 of 32 active), and took 39 us for any grid, however
+// small.  (512^2 39 -> 17 us, 4096^2 191 -> 174 us, 16384^2 2.64 -> 2.31 ms;
+// ten blocks an SM: 2.45 ms with eight, 2.25 with fourteen, which is slower
+// on the smaller grids.)
+// Each tile-local component is reduced to its maximum depth and the smallest
+// pixel attaining it, and every flat pixel takes its component's root.
+__global__ void __launch_bounds__(kCclThreads, 10)
+ccl_tile_kernel(int *__restrict__ L, unsigned long long *__restrict__ best,
+                LocalRoot *__restrict__ roots, int *__restrict__ nroots,
+                uint4 *__restrict__ edges, const int32_t *__restrict__ flats,
+                const float *__restrict__ orig, const float *__restrict__ filled, int64_t m,
+                int64_t n, int tm) {
+  __shared__ CclTile t;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tile = blockIdx.x;
+  const int64_t i0 = (int64_t)(tile % tm) * kTile, j0 = (int64_t)(tile / tm) * kTile;
+  const int64_t i = i0 + lane;  // pixels: lane = row, eight columns a warp
+  constexpr int kCols = kTile / (kCclThreads / 32);
+  bool some = false;
+  {
+    // every load of the thread in flight at once, from a clamped, always
+    // valid address
     const int64_t icl = i < m ? i : m - 1;
-    for (int j8 = 0; j8 < kTile; j8 += 8) {
-      int fv[8];
-      float fl[8], og[8];
+    int fv[kCols];
+    float fl[kCols], og[kCols];
 #pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int64_t j = j0 + j8 + u;
-        const int64_t p = (j < n ? j : n - 1) * m + icl;
-        fv[u] = flats[p];
-        fl[u] = filled[p];
-        og[u] = orig[p];
-      }
+    for (int u = 0; u < kCols; u++) {
+      const int64_t j = j0 + warp * kCols + u;
+      const int64_t p = (j < n ? j : n - 1) * m + icl;
+      fv[u] = flats[p];
+      fl[u] = filled[p];
+      og[u] = orig[p];
+    }
 #pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int jj = j8 + u;
-        const bool f = i < m && j0 + jj < n && (fv[u] & 1);
-        int k = INT_MIN;
-        if (f) {
-          const float d = __fsub_rn(fl[u], og[u]);
-          if (!isnan(d)) k = ordered_key(d);
-        }
-        t.key[jj * kTile + lane] = k;
-        t.root[jj * kTile + lane] = -1;
-        const uint32_t b = __ballot_sync(0xffffffffu, f);
-        if (lane == jj) my_mask = b;
-      }
-    }
-    {  // the tile's edge flat masks for the border pass: top and bottom row
-       // (bit = column), left and right column (bit = row)
-      const uint32_t top = __ballot_sync(0xffffffffu, my_mask & 1u);
-      const uint32_t bottom = __ballot_sync(0xffffffffu, (my_mask >> 31) & 1u);
-      const uint32_t left = __shfl_sync(0xffffffffu, my_mask, 0);
-      const uint32_t right = __shfl_sync(0xffffffffu, my_mask, kTile - 1);
-      if (lane == 0) edges[tile] = make_uint4(top, bottom, left, right);
-    }
-    // Tiles without flats (most of them) and tiles that are flat throughout
-    // (inside large flats) take short paths with the same results as the
-    // general one below.
-    const bool full = i0 + kTile <= m && j0 + kTile <= n;
-    if (!__any_sync(0xffffffffu, my_mask != 0)) {
-      __syncwarp();  // no labels: L is only ever read at flat pixels
-      continue;
-    }
-    if (full && __all_sync(0xffffffffu, my_mask == 0xffffffffu)) {
-      // one component; its root is run 0 (column 0, row 0) at pixel (i0, j0)
-      int kmax = INT_MIN;
-      for (int jj = 0; jj < kTile; jj++) kmax = max(kmax, t.key[jj * kTile + lane]);
-      kmax = __reduce_max_sync(0xffffffffu, kmax);
-      int first = INT_MAX;  // smallest tile index attaining the maximum
-      if (kmax != INT_MIN)
-        for (int jj = 0; jj < kTile; jj++)
-          if (t.key[jj * kTile + lane] == kmax) {
-            first = jj * kTile + lane;
-            break;
-          }
-      first = __reduce_min_sync(0xffffffffu, first);
-      const int64_t rootp = j0 * m + i0;
-      for (int jj = 0; jj < kTile; jj++) {
-        const int64_t gp = (j0 + jj) * m + i;
-        L[gp] = (int)rootp;
-        if (jj || lane) larg[gp] = -1;
-      }
-      if (lane == 0) {
-        lmax[rootp] = kmax;
-        larg[rootp] = first == INT_MAX
-                          ? INT_MAX
-                          : (int)((j0 + first / kTile) * m + (i0 + first % kTile));
-        best[rootp] = 0ULL;
-        roots[atomicAdd(nroots, 1)] = (int)rootp;
-      }
-      __syncwarp();
-      continue;
-    }
-    // lane = column c from here to the unions
-    const uint32_t M = my_mask, S = M & ~(M << 1);
-    t.starts[lane] = S;
-    for (uint32_t s = S; s; s &= s - 1) {
-      const int r = __ffs(s) - 1;
-      t.lab[lane * kTile + r] = lane * kTile + r;
-    }
-    __syncwarp();
-    const uint32_t M1 = __shfl_down_sync(0xffffffffu, M, 1);
-    const uint32_t S1 = __shfl_down_sync(0xffffffffu, S, 1);
-    if (lane < kTile - 1) {
-      for (uint32_t rs = S1; rs; rs &= rs - 1) {
-        const int s1 = __ffs(rs) - 1;
-        const uint32_t rm = run_mask(M1, s1);
-        uint32_t ov = M & (rm | (rm << 1) | (rm >> 1));
-        while (ov) {
-          const int s0 = run_start(S, __ffs(ov) - 1);
-          sunion(t.lab, lane * kTile + s0, (lane + 1) * kTile + s1);
-          ov &= ~run_mask(M, s0);
-        }
-      }
-    }
-    __syncwarp();
-    // lane = column: every pixel of a run takes the run's root, and the run
-    // parks its best (largest key, first pixel attaining it) at its start
-    for (uint32_t s = S; s; s &= s - 1) {
-      const int s0 = __ffs(s) - 1;
-      const int r = sfind(t.lab, lane * kTile + s0);
-      int km = INT_MIN, kl = 0;
-      for (uint32_t b = run_mask(M, s0); b; b &= b - 1) {
-        const int loc = lane * kTile + __ffs(b) - 1;
-        t.root[loc] = (int16_t)r;
-        const int k = t.key[loc];
-        if (k > km) {  // strictly: the first (smallest) pixel keeps a tie
-          km = k;
-          kl = loc;
-        }
-      }
-      t.key64[(lane * kTile + s0) >> 1] = km == INT_MIN ? 0ULL : pack_best(km, kl);
-    }
-    __syncwarp();
-    {  // local roots: clear their reduction slot and list them (one
-       // reservation per tile, lane = column)
-      uint32_t rs = 0;
-      for (uint32_t s = S; s; s &= s - 1) {
-        const int loc = lane * kTile + __ffs(s) - 1;
-        if (t.root[loc] == loc) {
-          t.lab64[loc >> 1] = 0ULL;
-          rs |= s & (~s + 1u);
-        }
-      }
-      const int mine = __popc(rs);
-      int incl = mine;
+    for (int q = 0; q < kSlotsPer; q++) t.lab[tid + q * kCclThreads] = tid + q * kCclThreads;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
+    for (int u = 0; u < kCols; u++) {
+      const int jj = warp * kCols + u;
+      const bool f = i < m && j0 + jj < n && (fv[u] & 1);
+      int k = INT_MIN;
+      if (f) {
+        const float d = __fsub_rn(fl[u], og[u]);
+        if (!isnan(d)) k = ordered_key(d);
       }
-      const int total = __shfl_sync(0xffffffffu, incl, 31);
-      int base = 0;
-      if (lane == 0 && total) base = atomicAdd(nroots, total);
-      base = __shfl_sync(0xffffffffu, base, 0) + incl - mine;
-      for (uint32_t b = rs; b; b &= b - 1)
-        roots[base++] = (int)((j0 + lane) * m + (i0 + __ffs(b) - 1));
+      t.key[jj * kTile + lane] = k;
+      const uint32_t b = __ballot_sync(0xffffffffu, f);
+      if (lane == 0) t.mask[jj] = b;
+      some |= f;
     }
-    __syncwarp();
-    // one 64-bit maximum per run folds its best into its root
-    for (uint32_t s = S; s; s &= s - 1) {
-      const int loc = lane * kTile + __ffs(s) - 1;
-      const unsigned long long v = t.key64[loc >> 1];
-      if (v) atomicMax(&t.lab64[t.root[loc] >> 1], v);
+  }
+  some = __syncthreads_or(some);
+  if (warp == 0) {  // the tile's edge flat masks for the border pass: top and
+                    // bottom row (bit = column), left and right column (bit = row)
+    const uint32_t mk = t.mask[lane];
+    const uint32_t top = __ballot_sync(0xffffffffu, mk & 1u);
+    const uint32_t bottom = __ballot_sync(0xffffffffu, (mk >> 31) & 1u);
+    if (lane == 0) edges[tile] = make_uint4(top, bottom, t.mask[0], t.mask[kTile - 1]);
+  }
+  if (!some) return;  // no labels: L is only ever read at flat pixels
+
+#pragma unroll
+  for (int q = 0; q < kSlotsPer; q++) {  // unions with the column before
+    const int slot = tid + q * kCclThreads, c = slot >> 4;
+    const uint32_t M = t.mask[c];
+    const int s0 = slot_row(run_starts(M), slot & 15);
+    if (s0 < 0 || c == 0) continue;
+    const uint32_t M1 = t.mask[c - 1], S1 = run_starts(M1);
+    const uint32_t rm = run_mask(M, s0);
+    uint32_t ov = M1 & (rm | (rm << 1) | (rm >> 1));
+    while (ov) {
+      const int s1 = run_start(S1, __ffs(ov) - 1);
+      sunion(t.lab, (c - 1) * 16 + (s1 >> 1), slot);
+      ov &= ~run_mask(M1, s1);
     }
-    __syncwarp();
-    // lane = row: labels and the roots' maximum / argmax, coalesced per column
-    for (int jj = 0; jj < kTile; jj++) {
-      const int64_t j = j0 + jj;
-      const bool in = i < m && j < n;
-      const int64_t gp = j * m + i;
-      const int loc = jj * kTile + lane;
-      const int r = t.root[loc];
-      if (!in || r < 0) continue;  // L is only ever read at flat pixels
-      if (r == loc) {
-        const unsigned long long v = t.lab64[loc >> 1];
-        const int a = 1023 - (int)(v & 1023u);
-        lmax[gp] = v ? (int)((unsigned)(v >> 32) ^ 0x80000000u) : INT_MIN;
-        larg[gp] = v ? (int)((j0 + a / kTile) * m + (i0 + a % kTile)) : INT_MAX;
-        best[gp] = 0ULL;
-      } else {
-        larg[gp] = -1;  // not a local root
+  }
+  __syncthreads();
+
+  // Every run finds its root and its best (largest key, first pixel attaining
+  // it); roots start the reduction with their own.
+  unsigned long long mine[kSlotsPer];
+  int root[kSlotsPer], nroot = 0;
+#pragma unroll
+  for (int q = 0; q < kSlotsPer; q++) {
+    const int slot = tid + q * kCclThreads, c = slot >> 4;
+    const uint32_t M = t.mask[c];
+    const int s0 = slot_row(run_starts(M), slot & 15);
+    root[q] = -1;
+    mine[q] = 0ULL;
+    if (s0 < 0) continue;
+    root[q] = sfind(t.lab, slot);
+    int km = INT_MIN, kl = 0;
+    for (uint32_t b = run_mask(M, s0); b; b &= b - 1) {
+      const int loc = c * kTile + __ffs(b) - 1;
+      const int k = t.key[loc];
+      if (k > km) {  // strictly: the first (smallest) pixel keeps a tie
+        km = k;
+        kl = loc;
       }
-      L[gp] = (int)((j0 + r / kTile) * m + (i0 + r % kTile));
     }
-    __syncwarp();
+    if (km != INT_MIN) mine[q] = pack_best(km, kl);
+    if (root[q] == slot) {
+      t.best[slot] = mine[q];
+      nroot++;
+    }
+  }
+  int incl = nroot;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) t.warp_roots[warp] = incl;
+  __syncthreads();
+  if (tid == 0) {  // one reservation per tile in the list of local roots
+    int total = 0;
+    for (int w = 0; w < kCclThreads / 32; w++) total += t.warp_roots[w];
+    t.base = atomicAdd(nroots, total);
+  }
+#pragma unroll
+  for (int q = 0; q < kSlotsPer; q++) {
+    const int slot = tid + q * kCclThreads;
+    if (root[q] < 0) continue;
+    if (root[q] != slot) {
+      t.lab[slot] = root[q];  // for the pixels below
+      if (mine[q]) atomicMax(&t.best[root[q]], mine[q]);
+    }
+  }
+  __syncthreads();
+
+  int at = t.base + incl - nroot;
+  for (int w = 0; w < warp; w++) at += t.warp_roots[w];
+#pragma unroll
+  for (int q = 0; q < kSlotsPer; q++) {
+    const int slot = tid + q * kCclThreads, c = slot >> 4;
+    if (root[q] != slot) continue;
+    const int gp = (int)((j0 + c) * m + i0 + slot_row(run_starts(t.mask[c]), slot & 15));
+    const unsigned long long v = t.best[slot];
+    const int a = 1023 - (int)(v & 1023u);
+    roots[at++] = LocalRoot{gp, v ? (int)((unsigned)(v >> 32) ^ 0x80000000u) : INT_MIN,
+                            v ? (int)((j0 + a / kTile) * m + (i0 + a % kTile)) : INT_MAX, 0};
+    best[gp] = 0ULL;
+  }
+#pragma unroll
+  for (int u = 0; u < kCols; u++) {  // labels, coalesced per column
+    const int jj = warp * kCols + u;
+    const uint32_t M = t.mask[jj];
+    if (!((M >> lane) & 1u)) continue;  // L is only ever read at flat pixels
+    const int r = t.lab[jj * 16 + (run_start(run_starts(M), lane) >> 1)];
+    const int rc = r >> 4;
+    L[(j0 + jj) * m + i] =
+        (int)((j0 + rc) * m + i0 + slot_row(run_starts(t.mask[rc]), r & 15));
   }
 }
 
@@ -405,17 +381,15 @@ __device__ __forceinline__ int root_arg(unsigned long long v) {
 // above a pixel is a local root).  The roots are final here (every union
 // is done), and a label only ever moves down to the root, so pointing a
 // local root at it while other threads still walk through it is safe.
-__global__ void ccl_root_kernel(int *__restrict__ L, const int *__restrict__ lmax,
-                                const int *__restrict__ larg, const int *__restrict__ roots,
+__global__ void ccl_root_kernel(int *__restrict__ L, const LocalRoot *__restrict__ roots,
                                 const int *__restrict__ nroots,
                                 unsigned long long *__restrict__ best) {
   const int K = *nroots;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) {
-    const int p = roots[k];
-    const int R = uf_find(L, p);
-    const int key = lmax[p];
-    if (key != INT_MIN) atomicMax(&best[R], pack_root(key, larg[p]));
-    atomicMin(&L[p], R);
+    const int4 r = __ldg(reinterpret_cast<const int4 *>(roots + k));  // pixel, key, arg
+    const int R = uf_find(L, r.x);
+    if (r.y != INT_MIN) atomicMax(&best[R], pack_root(r.y, r.z));
+    atomicMin(&L[r.x], R);
   }
 }
 
@@ -503,25 +477,23 @@ tt_cuda_status costs_dev(float *costs, ptrdiff_t *conncomps,
   const int64_t N = g.cells();
   Workspace &ws = workspace();
   const int T = g.tiles();
-  if (!ws.reserve(4 * align_up((size_t)N * 4) + align_up((size_t)N * 8) +
-                  align_up((size_t)T * 16) + 256))
+  const size_t nr = std::min((size_t)N, (size_t)T * kMaxRoots);
+  if (!ws.reserve(align_up((size_t)N * 4) + align_up((size_t)N * 8) +
+                  align_up(nr * sizeof(LocalRoot)) + align_up((size_t)T * 16) + 256))
     return TT_CUDA_ERR_ALLOC;
   int *nroots = (int *)ws.take(256);
   uint4 *edges = (uint4 *)ws.take((size_t)T * 16);
-  int *roots = (int *)ws.take((size_t)N * 4);
+  LocalRoot *roots = (LocalRoot *)ws.take(nr * sizeof(LocalRoot));
   int *L = (int *)ws.take((size_t)N * 4);
-  int *lmax = (int *)ws.take((size_t)N * 4);
-  int *larg = (int *)ws.take((size_t)N * 4);
   unsigned long long *best = (unsigned long long *)ws.take((size_t)N * 8);
   const int grid = ew_grid(N);
-  // one tile per warp: the block scheduler evens out tiles whose labelling
-  // takes longer (many runs, many unions)
-  const int tgrid = (int)std::min<int64_t>((T + kCclWarps - 1) / kCclWarps, INT_MAX);
   TT_CHECK(cudaMemsetAsync(nroots, 0, sizeof(int), st));
-  TT_LAUNCH(ccl_tile_kernel, tgrid, kCclWarps * 32, 0, st, L, lmax, larg, best, roots,
-            nroots, edges, flats, orig, filled, g.m, g.n, g.tm, g.tn);
+  // one tile per block: the block scheduler evens out tiles whose labelling
+  // takes longer (many runs, many unions)
+  TT_LAUNCH(ccl_tile_kernel, T, kCclThreads, 0, st, L, best, roots, nroots, edges, flats, orig,
+            filled, g.m, g.n, g.tm);
   TT_LAUNCH(ccl_border_kernel, (T + 7) / 8, 256, 0, st, L, edges, g.m, g.tm, g.tn);
-  TT_LAUNCH(ccl_root_kernel, grid, 256, 0, st, L, lmax, larg, roots, nroots, best);
+  TT_LAUNCH(ccl_root_kernel, grid, 256, 0, st, L, roots, nroots, best);
   const int cgrid = (int)std::min<int64_t>((N + 1023) / 1024, (int64_t)sm_count() * 32);
   if (seed)
     TT_LAUNCH(costs_kernel<true>, cgrid, 256, 0, st, costs, conncomps, L, best,
