@@ -109,7 +109,9 @@ struct RelaxArgs {
   int64_t m, n;
   int tm, tn;
   QueueCtl *ctl;
-  int *dirty;  // per tile: nonzero while waiting to be relaxed
+  const int *start;  // per tile: nonzero where the tile starts dirty (nullptr: every tile)
+  int *words;        // dirty words, by owner (see word_of), zeroed
+  int per_warp;      // word slots of a warp: its tiles, rounded up to whole sectors
   unsigned long long max_visits;
   int visit_flush;  // a warp adds its visits to ctl->visits in batches of this
   int *prio;        // ordered schedules: per tile, the key of the lowest value
@@ -117,6 +119,19 @@ struct RelaxArgs {
   int *wmin;        // ordered schedules: per warp, the lowest priority among
                     // its waiting tiles at its last pass (kClean: none)
 };
+
+// Tile k * W + w is warp w's k-th and has word w * per_warp + k: a warp's
+// words lie together, so a poll reads its tiles' state in a few sectors
+// instead of one for each tile (4096^2: 1 instead of 6, 16384^2: 11 instead
+// of 87; fill 5.96 -> 5.66 ms, gwdt 9.8 -> 9.1 ms at 16384^2).
+constexpr int kSectorInts = 8;
+__host__ __device__ __forceinline__ int words_per_warp(int tiles, int warps) {
+  return ((tiles + warps - 1) / warps + kSectorInts - 1) / kSectorInts * kSectorInts;
+}
+__device__ __forceinline__ int word_of(const RelaxArgs &a, int tile, int W) {
+  const unsigned k = (unsigned)tile / (unsigned)W;
+  return (int)((unsigned)tile - k * W) * a.per_warp + (int)k;
+}
 
 // Order-preserving integer key of a float (key order == value order).
 __device__ __forceinline__ int value_key(float x) {
@@ -462,10 +477,16 @@ __device__ bool raise_threshold(const RelaxArgs &a, int lane, int W, int thr) {
 // With every warp idle (idle word `seen`): finish the run if no flag is set
 // and no warp has woken since.  A warp leaves the idle count before it takes
 // a word down, so a flag that is gone shows in the count.
-__device__ void check_done(const RelaxArgs &a, int lane, int T, unsigned long long seen) {
+__device__ void check_done(const RelaxArgs &a, int lane, int n, unsigned long long seen) {
   fence_acq_rel_gpu();  // every flag set before its warp went idle is visible
   bool any = false;
-  for (int t = lane; t < T; t += 32) any |= *(volatile int *)&a.dirty[t] != 0;
+  // per_warp is a multiple of eight: sixteen bytes a load
+  const int4 *const w = reinterpret_cast<const int4 *>(a.words);
+#pragma unroll 8
+  for (int t = lane; t < n / 4; t += 32) {
+    const int4 v = __ldcv(w + t);
+    any |= (v.x | v.y | v.z | v.w) != 0;
+  }
   if (__any_sync(0xffffffffu, any) || lane != 0) return;
   fence_acq_rel_gpu();
   if (*(volatile unsigned long long *)&a.ctl->idle == seen) atomicExch(&a.ctl->done, 1);
@@ -486,6 +507,15 @@ relax_persistent_kernel(RelaxArgs a) {
   unsigned long long unflushed = 0;  // visits not yet added to ctl
   int posted = kClean;               // ordered: this warp's last wmin entry
   int raised_at = kUrgent;           // ordered: threshold this warp last raised from
+  const int own = wid < T ? (T - wid + W - 1) / W : 0;  // tiles of this warp
+  int *const words = a.words + (size_t)wid * a.per_warp;
+  for (int k = lane; k < own; k += 32) {  // the tiles that start dirty
+    const int tile = wid + k * W;
+    const int f = a.start ? a.start[tile] : DIRTY_FULL;
+    if (ordered_sched(SCHED) && !a.start) a.prio[tile] = kUrgent;
+    if (f) atomicAdd(&words[k], f);  // (neighbours may publish already)
+  }
+  __syncwarp();
   for (;;) {
     // The control words and the first flags are loaded together: a poll
     // costs one round trip to L2, which is on the path of every change that
@@ -493,7 +523,7 @@ relax_persistent_kernel(RelaxArgs a) {
     unsigned long long idle_word, stop_word;
     asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];"
                  : "=l"(idle_word), "=l"(stop_word) : "l"(a.ctl) : "memory");
-    const int f0 = wid + lane * W < T ? *(volatile int *)&a.dirty[wid + lane * W] : 0;
+    const int f0 = lane < own ? *(volatile int *)&words[lane] : 0;
     const int thr = ordered_sched(SCHED) ? *(volatile int *)&a.ctl->thresh : 0;
     if (stop_word) break;
     int lane_wait = kClean;  // ordered: lowest priority of this lane's waiting tiles
@@ -503,10 +533,10 @@ relax_persistent_kernel(RelaxArgs a) {
       unflushed = 0;
     }
     int taken = 0;
-    for (int base = wid; base < T && taken < kTakeTiles; base += W * 32) {
-      const int mine = base + lane * W;
+    for (int base = 0; base < own && taken < kTakeTiles; base += 32) {
+      const int mine = wid + (base + lane) * W;
       int f = f0;
-      if (base != wid) f = (mine < T) ? *(volatile int *)&a.dirty[mine] : 0;
+      if (base) f = base + lane < own ? *(volatile int *)&words[base + lane] : 0;
       bool elig = f != 0;
       if (ordered_sched(SCHED) && elig) {
         const int pr = *(volatile int *)&a.prio[mine];
@@ -525,9 +555,9 @@ relax_persistent_kernel(RelaxArgs a) {
       while (mask && taken < kTakeTiles) {
         const int l = __ffs(mask) - 1;
         mask &= mask - 1;
-        const int tile = base + l * W;
+        const int tile = wid + (base + l) * W;
         if (taken) {  // earlier visits took time: what is pending now
-          if (lane == l) f = *(volatile int *)&a.dirty[tile];
+          if (lane == l) f = *(volatile int *)&words[base + l];
           fence_acq_rel_gpu();
         }
         const int got = __shfl_sync(0xffffffffu, f, l);
@@ -540,7 +570,7 @@ relax_persistent_kernel(RelaxArgs a) {
         if (woke && !fenced) fence_acq_rel_gpu();
         woke = false;
         __syncwarp();
-        if (lane == l) atomicSub(&a.dirty[tile], got);  // the lane that polls this word
+        if (lane == l) atomicSub(&words[base + l], got);  // the lane that polls this word
       }
     }
     int wait_min = kClean;
@@ -566,9 +596,9 @@ relax_persistent_kernel(RelaxArgs a) {
         fence_acq_rel_gpu();
         raised_at = thr;
         if (!raise_threshold<SCHED>(a, lane, W, thr) && wid == 0)
-          check_done(a, lane, T, idle_word);
+          check_done(a, lane, W * a.per_warp, idle_word);
       } else if (!ordered_sched(SCHED) && wid == 0) {
-        check_done(a, lane, T, idle_word);
+        check_done(a, lane, W * a.per_warp, idle_word);
       }
     }
     int stop = 0;
@@ -576,12 +606,16 @@ relax_persistent_kernel(RelaxArgs a) {
       if (++spins > kSpinLimit) {
         atomicOr(&a.ctl->abort, ABORT_SPIN);
         stop = 1;
-      } else if ((T > W && wid != 0) || spins > 4096) {
-        // a warp that owns one tile waits on one flag, and warp 0 ends the
-        // run: they poll at once.  The others' polls take issue slots and L2
-        // accesses from the warps at work (64 to 512 ns between them instead:
-        // 4096^2 1.04 / 2.27 against 1.01 / 2.23 ms).
-        __nanosleep(1000);
+      } else if (((T > W || KIND != FILL) && wid != 0) || spins > 4096) {
+        // Warp 0, which ends the run, and a fill's warps with one tile each
+        // poll at once.  The others sleep: the polls of idle warps take issue
+        // slots from the warps at work, and on gwdt, whose tiles are visited
+        // again when a shorter path comes in, a warp that looks later takes
+        // in more changes at once (4096^2 / 16384^2 ms at 50 ns 2.43 / 9.26,
+        // 1 us 2.21 / 9.13, 4 us 2.11 / 8.96, 16 us 2.17 / 8.91, fill 1.05 /
+        // 5.70, 1.01 / 5.66, 1.04 / 5.68, 1.51 / 5.98; 2048 x 1500, a tile a
+        // warp, gwdt 0.69 ms at once, 0.61 at 0.8 us).
+        __nanosleep(KIND == FILL ? 1000 : T > W ? 4000 : 800);
       }
     }
     if (__shfl_sync(0xffffffffu, stop, 0)) break;
@@ -803,7 +837,7 @@ __device__ bool relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
       fenced = true;
       if (tgt >= 0) {
         if (ordered_sched(SCHED)) atomicMin(&a.prio[tgt], key);
-        atomicAdd(&a.dirty[tgt], val);
+        atomicAdd(&a.words[word_of(a, tgt, gridDim.x * kWarps)], val);
       }
     }
     if (done || sweeps >= kCap) break;
@@ -1033,14 +1067,6 @@ __global__ void negate_kernel(float *__restrict__ out, const float *__restrict__
     out[p] = -in[p];
 }
 
-// Mark every tile dirty (fill starts everywhere), most urgent.
-__global__ void dirty_all_kernel(int *dirty, int *prio, int n) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    dirty[t] = DIRTY_FULL;
-    if (prio) prio[t] = kUrgent;
-  }
-}
-
 // gwdt working arrays: distance 1 at presills, +INF at other flats and 0
 // at non-flat pixels, as src/gwdt.c:296-308 starts.  Non-flat pixels take
 // cost NaN for the run: every path through one and every update of one
@@ -1049,7 +1075,7 @@ __global__ void dirty_all_kernel(int *dirty, int *prio, int n) {
 __global__ void gwdt_init_kernel(float *__restrict__ dist, float *__restrict__ wcost,
                                  const float *__restrict__ costs,
                                  const int32_t *__restrict__ flats, int64_t m,
-                                 int64_t n, RelaxArgs qa) {
+                                 int64_t n, RelaxArgs qa, int *__restrict__ dirty) {
   const int64_t N = m * n;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p0 < N; p0 += kEw * stride) {
@@ -1068,7 +1094,7 @@ __global__ void gwdt_init_kernel(float *__restrict__ dist, float *__restrict__ w
       const int32_t f = fv[u];
       dist[p] = (f & 5) == 5 ? 1.0f : (f & 1) ? INFINITY : 0.0f;
       wcost[p] = (f & 1) ? cv[u] : NAN;
-      if ((f & 5) == 5) mark_tiles_around(qa.dirty, qa.prio, qa.tm, p % m, p / m, m, n);
+      if ((f & 5) == 5) mark_tiles_around(dirty, qa.prio, qa.tm, p % m, p / m, m, n);
     }
   }
 }
@@ -1167,6 +1193,26 @@ cudaError_t launch_relax(int grid, const RelaxArgs &ra, cudaStream_t st) {
   return cudaLaunchKernelEx(&cfg, relax_persistent_kernel<KIND, SCHED>, ra);
 }
 
+// Blocks of a relaxation over T tiles: every SM full, but no more warps than
+// tiles (each warp owns at least one).
+template <int KIND>
+int relax_grid(int sched, int T) {
+  static int blocks_per_sm[3][kSchedules] = {};
+  if (!blocks_per_sm[KIND][sched]) {
+    int b = 0;
+    switch (sched) {
+      case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<KIND, 1>, kWarps * 32, 0); break;
+      case 2: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<KIND, 2>, kWarps * 32, 0); break;
+      case 3: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<KIND, 3>, kWarps * 32, 0); break;
+      case 4: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<KIND, 4>, kWarps * 32, 0); break;
+      case 5: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<KIND, 5>, kWarps * 32, 0); break;
+      default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<KIND, 0>, kWarps * 32, 0); break;
+    }
+    blocks_per_sm[KIND][sched] = b > 0 ? b : 1;
+  }
+  return std::max(1, std::min(sm_count() * blocks_per_sm[KIND][sched], (T + kWarps - 1) / kWarps));
+}
+
 // Host driver: mark the starting tiles, run one persistent launch, read the
 // status.  `bc` (sink filling only) selects the seeded start: the fill's
 // initial state is written here and only tiles next to a seed start dirty;
@@ -1183,11 +1229,15 @@ tt_cuda_status run_queue(float *state, const float *aux, const int32_t *flats,
   // gwdt seeded by the costs pass: state, costs and flags are in place
   const bool seeded = KIND != FILL && seeded_dirty;
   if (seeded && ordered) return TT_CUDA_ERR_INVALID_ARGUMENT;  // no priorities seeded
-  const int wmax = sm_count() * 32 * kWarps;  // more warp slots than any grid has warps
+  const int grid = relax_grid<KIND>(sched, T);
+  const int W = grid * kWarps, per_warp = words_per_warp(T, W);
+  const size_t words_bytes = (size_t)W * per_warp * 4;
+  // a fill without seeds starts everywhere and needs no flags
+  const bool all = KIND == FILL && !bc;
   Workspace &ws = workspace();
-  size_t need = align_up(sizeof(QueueCtl)) + align_up((size_t)T * 4);
+  size_t need = align_up(sizeof(QueueCtl)) + align_up((size_t)T * 4) + align_up(words_bytes);
   if (KIND != FILL && !seeded) need += align_up((size_t)g.cells() * 4);
-  if (ordered) need += align_up((size_t)T * 4) + align_up((size_t)wmax * 4);
+  if (ordered) need += align_up((size_t)T * 4) + align_up((size_t)W * 4);
   if (!ws.reserve(need)) return TT_CUDA_ERR_ALLOC;
   // inside a pipeline call the control block and the flags come cleared
   CallArena *const arena = call_arena();
@@ -1196,29 +1246,36 @@ tt_cuda_status run_queue(float *state, const float *aux, const int32_t *flats,
                                         : arena->zeroed(sizeof(QueueCtl)));
   const bool in_arena = ctl != nullptr;
   if (!ctl) ctl = (QueueCtl *)ws.take(sizeof(QueueCtl));
-  int *dirty = seeded ? seeded_dirty : arena ? (int *)arena->zeroed((size_t)T * 4) : nullptr;
-  const bool dirty_clear = dirty != nullptr;
-  if (!dirty) dirty = (int *)ws.take((size_t)T * 4);
+  auto cleared = [&](size_t bytes) -> int * {  // arena memory, else memory to clear
+    return arena ? (int *)arena->zeroed(bytes) : nullptr;
+  };
+  int *dirty = all ? nullptr : seeded ? seeded_dirty : cleared((size_t)T * 4);
+  const bool dirty_clear = all || dirty != nullptr;
+  if (!dirty_clear) dirty = (int *)ws.take((size_t)T * 4);
+  int *words = cleared(words_bytes);
+  const bool words_clear = words != nullptr;
+  if (!words) words = (int *)ws.take(words_bytes);
   // gwdt relaxes over a copy of the costs with NaN at non-flat pixels (a
   // seeded run over the costs array itself, already in that form)
   float *wcost = KIND == FILL ? nullptr
                  : seeded    ? const_cast<float *>(aux)
                              : (float *)ws.take((size_t)g.cells() * 4);
   int *prio = ordered ? (int *)ws.take((size_t)T * 4) : nullptr;
-  int *wmin = ordered ? (int *)ws.take((size_t)wmax * 4) : nullptr;
+  int *wmin = ordered ? (int *)ws.take((size_t)W * 4) : nullptr;
   QueueCtl *hctl = (QueueCtl *)pinned_scratch();
   if (!hctl) return TT_CUDA_ERR_ALLOC;
 
-  RelaxArgs ra{state, KIND != FILL ? wcost : aux, g.m, g.n, g.tm, g.tn, ctl, dirty, 0, 1,
-               prio, wmin};
+  RelaxArgs ra{state, KIND != FILL ? wcost : aux, g.m, g.n, g.tm, g.tn, ctl, dirty, words,
+               per_warp, 0, 1, prio, wmin};
   if (ordered) {  // no priorities, no waiting work (kClean = 0x7f7f7f7f)
     TT_CHECK(cudaMemsetAsync(prio, 0x7f, (size_t)T * 4, st));
-    TT_CHECK(cudaMemsetAsync(wmin, 0x7f, (size_t)wmax * 4, st));
+    TT_CHECK(cudaMemsetAsync(wmin, 0x7f, (size_t)W * 4, st));
   }
   const int64_t cap_rounds = max_rounds();
   ra.max_visits = (unsigned long long)T * (unsigned long long)std::min<int64_t>(cap_rounds, 1LL << 20);
   if (!in_arena) TT_CHECK(cudaMemsetAsync(ctl, 0, sizeof(QueueCtl), st));
   if (!dirty_clear) TT_CHECK(cudaMemsetAsync(dirty, 0, (size_t)T * 4, st));
+  if (!words_clear) TT_CHECK(cudaMemsetAsync(words, 0, words_bytes, st));
   const int tgrid = (T + 255) / 256;
   if (KIND == FILL && bc && bound) {
     if (g.m % kCoarse == 0 && aligned16(state) && aligned16(aux) && aligned4(bc))
@@ -1233,30 +1290,12 @@ tt_cuda_status run_queue(float *state, const float *aux, const int32_t *flats,
   } else if (KIND == FILL && bc) {
     TT_LAUNCH(fill_init_kernel, elementwise_grid(g.cells()), 256, 0, st, state, aux, bc, g.m,
               g.n, dirty, prio, g.tm);
-  } else if (KIND == FILL) {
-    TT_LAUNCH(dirty_all_kernel, tgrid, 256, 0, st, dirty, prio, T);
-  } else if (!seeded) {
+  } else if (KIND != FILL && !seeded) {
     TT_LAUNCH(gwdt_init_kernel, elementwise_grid(g.cells()), 256, 0, st, state, wcost, aux,
-              flats, g.m, g.n, ra);
+              flats, g.m, g.n, ra, dirty);
   }
   TT_CHECK(cudaGetLastError());
-  static int blocks_per_sm[3][kSchedules] = {};
-  if (!blocks_per_sm[KIND][sched]) {
-    int b = 0;
-    switch (sched) {
-      case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<KIND, 1>, kWarps * 32, 0); break;
-      case 2: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<KIND, 2>, kWarps * 32, 0); break;
-      case 3: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<KIND, 3>, kWarps * 32, 0); break;
-      case 4: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<KIND, 4>, kWarps * 32, 0); break;
-      case 5: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<KIND, 5>, kWarps * 32, 0); break;
-      default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<KIND, 0>, kWarps * 32, 0); break;
-    }
-    blocks_per_sm[KIND][sched] = b > 0 ? b : 1;
-  }
-  // No more warps than tiles (each warp owns at least one tile).
-  int grid = sm_count() * blocks_per_sm[KIND][sched];
-  grid = std::max(1, std::min(grid, (T + kWarps - 1) / kWarps));
-  ra.visit_flush = visit_flush(ra.max_visits, grid * kWarps);
+  ra.visit_flush = visit_flush(ra.max_visits, W);
   switch (sched) {
     case 1: TT_CHECK((launch_relax<KIND, 1>(grid, ra, st))); break;
     case 2: TT_CHECK((launch_relax<KIND, 2>(grid, ra, st))); break;
@@ -1357,9 +1396,9 @@ tt_cuda_status gwdt_dev(float *dist, ptrdiff_t *prev, const float *costs,
 // For callers that cannot allocate device memory once they are running: a
 // framework whose own pool already holds the device's memory, or a loop
 // that must not pay for cudaMalloc/cudaFree (both can synchronise the whole
-// device).  The only scratch of the fill -- the control block and one flag
-// per 32 x 32 tile -- lives in the file-scope array below, sized for
-// kNoAllocMaxTiles tiles; every device that loads this library holds it
+// device).  The only scratch of the fill -- the control block and one word
+// per 32 x 32 tile, rounded up for each warp -- lives in the file-scope array
+// below, sized for kNoAllocMaxTiles tiles; every device that loads this library holds it
 // until the process exits.  All calls share it: each call clears what must
 // start at zero, and calls that overlap on the GPU race on it.  The array's
 // device address is looked up once per device and kept; a caller that
@@ -1367,8 +1406,10 @@ tt_cuda_status gwdt_dev(float *dist, ptrdiff_t *prev, const float *costs,
 // call this entry point afterwards in the same process.
 // ------------------------------------------------------------------
 constexpr int kNoAllocMaxTiles = 65536;  // e.g. 8192 x 8192 pixels
+constexpr int kNoAllocMaxWarps = 8192;   // whose words are rounded up to whole sectors
 constexpr int kNoAllocHeaderWords = 64;  // control block, padded to 256 bytes
-static __device__ __align__(256) int g_fill_scratch[kNoAllocHeaderWords + kNoAllocMaxTiles];
+static __device__ __align__(256) int
+    g_fill_scratch[kNoAllocHeaderWords + kNoAllocMaxTiles + kNoAllocMaxWarps * kSectorInts];
 
 namespace {
 void *g_fill_scratch_addr[64];  // device address of g_fill_scratch, per device
@@ -1402,22 +1443,19 @@ tt_cuda_status fill_noalloc(float *f, const float *dem, const uint8_t *bc,
   tt_cuda_status s = fill_scratch_address(&base);
   if (s != TT_CUDA_SUCCESS) return s;
   QueueCtl *ctl = (QueueCtl *)base;
-  int *dirty = (int *)base + kNoAllocHeaderWords;
+  int *words = (int *)base + kNoAllocHeaderWords;
   const int T = g.tiles();
+  const int grid = std::min(relax_grid<FILL>(0, T), kNoAllocMaxWarps / kWarps);
+  const int W = grid * kWarps, per_warp = words_per_warp(T, W);
   TT_LAUNCH(fill_init_kernel, elementwise_grid(g.cells()), 256, 0, st, f, dem, bc, g.m,
             g.n, nullptr, nullptr, g.tm);
-  TT_CHECK(cudaMemsetAsync(ctl, 0, sizeof(QueueCtl), st));
-  TT_LAUNCH(dirty_all_kernel, (T + 255) / 256, 256, 0, st, dirty, (int *)nullptr, T);
+  TT_CHECK(cudaMemsetAsync(ctl, 0, (kNoAllocHeaderWords + (size_t)W * per_warp) * 4, st));
   TT_CHECK(cudaGetLastError());
-  RelaxArgs ra{f, dem, g.m, g.n, g.tm, g.tn, ctl, dirty, 0, 1, nullptr, nullptr};
+  RelaxArgs ra{f, dem, g.m, g.n, g.tm, g.tn, ctl, nullptr, words, per_warp, 0, 1, nullptr,
+               nullptr};
   ra.max_visits = (unsigned long long)T *
                   (unsigned long long)std::min<int64_t>(max_rounds(), 1LL << 20);
-  int b = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, relax_persistent_kernel<FILL, 0>,
-                                                kWarps * 32, 0);
-  int grid = sm_count() * (b > 0 ? b : 1);
-  grid = std::max(1, std::min(grid, (T + kWarps - 1) / kWarps));
-  ra.visit_flush = visit_flush(ra.max_visits, grid * kWarps);
+  ra.visit_flush = visit_flush(ra.max_visits, W);
   TT_CHECK((launch_relax<FILL, 0>(grid, ra, st)));
   QueueCtl h;  // read back into host stack memory: no pinned allocation
   TT_CHECK(cudaMemcpyAsync(&h, ctl, sizeof(QueueCtl), cudaMemcpyDeviceToHost, st));

@@ -2,6 +2,7 @@
 // workspaces and call locks, and the public entry points of
 // include/tt_cuda.h.  Host-pointer entry points stage their arrays through
 // device buffers and call the device-pointer stage functions.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -131,8 +132,12 @@ ArenaScope::~ArenaScope() { g_arena = prev_; }
 constexpr size_t kBlockBytes = kBlockInts * sizeof(int);
 
 size_t CallArena::bytes(int tiles) {
-  // tile flags of the fill, of its coarser starts and of gwdt
-  return kArenaBlocks * kBlockBytes + 3 * (align_up((size_t)tiles * 4) + 1024);
+  // tile flags of the fill, of its coarser starts and of gwdt, and the same
+  // once more for the words by owner, which a warp rounds up by eight ints
+  // at most (a run has no more warps than tiles, nor than fill the SMs)
+  const size_t warps = std::min<size_t>(tiles, (size_t)sm_count() * 32) + 4;
+  return kArenaBlocks * kBlockBytes +
+         3 * (2 * align_up((size_t)tiles * 4) + align_up(warps * 32) + 1024);
 }
 
 tt_cuda_status CallArena::init(void *base, int tiles, cudaStream_t st) {
