@@ -30,7 +30,9 @@
 // with a ballot); a warp that relaxes a tile marks a neighbouring tile dirty
 // when one of its new values would lower a pixel there, so information
 // crosses tile borders as soon as a tile finishes, with no host round trips
-// and no shared queue to contend on.
+// and no shared queue to contend on.  Among its own dirty tiles a warp takes
+// those into which the lowest values came first; warps do not wait for one
+// another's values (the ordered schedules below do).
 // A tile has a single owner, so no two warps relax it at once.
 //
 // Termination: only a running warp sets flags.  A warp that finds none of
@@ -58,14 +60,14 @@ namespace {
 
 constexpr int kWarps = 4;        // tiles per block
 constexpr int kMaxSweeps = 256;  // per tile visit; a capped tile re-enqueues
-// Tiles a warp relaxes before it looks at its flags again from its lowest
-// tile on.  Few keep the warps together in one region of a large grid, whose
-// tiles are still in L2 when they are visited again; too few, and a region is
-// relaxed too far on what it knows and visited more often.  16384^2: fill
-// 8.2 ms with all 32 of a poll, 6.4 with four, 6.1 with two, 6.4 with one;
-// gwdt 12.1 with all, 10.3 with 16, 10.1 with eight, 9.9 with four, 10.6
-// with two.
-constexpr int kTakeFill = 2, kTakeGwdt = 4;
+// Tiles a warp relaxes before it looks at all its words again.  It takes its
+// waiting tiles in the order of the lowest value published into them, which
+// leaves fewer of them to be visited again when a lower one comes in.  fill /
+// gwdt ms in the order of the tiles (two / four at a time), and by value with
+// one, two, three and four (gwdt) at a time: 16384^2 5.66 / 8.96, then gwdt
+// 8.46, 8.50, -, 8.93 and fill 5.63, 5.60, 5.59; 4096^2 1.01 / 2.06, 0.93 /
+// 1.86 with three / two; 64 DEMs in a batch 0.48 / 0.75, 0.44 / 0.69.
+constexpr int kTakeFill = 3, kTakeGwdt = 2;
 
 constexpr float kSqrt2 = 1.41421356237309504880f;
 
@@ -112,6 +114,8 @@ struct RelaxArgs {
   const int *start;  // per tile: nonzero where the tile starts dirty (nullptr: every tile)
   int *words;        // dirty words, by owner (see word_of), zeroed
   int per_warp;      // word slots of a warp: its tiles, rounded up to whole sectors
+  unsigned *keys;    // beside the words, zeroed: the inverted key of the lowest value
+                     // published into the tile since it was taken (0: none)
   unsigned long long max_visits;
   int visit_flush;  // a warp adds its visits to ctl->visits in batches of this
   int *prio;        // ordered schedules: per tile, the key of the lowest value
@@ -509,11 +513,15 @@ relax_persistent_kernel(RelaxArgs a) {
   int raised_at = kUrgent;           // ordered: threshold this warp last raised from
   const int own = wid < T ? (T - wid + W - 1) / W : 0;  // tiles of this warp
   int *const words = a.words + (size_t)wid * a.per_warp;
+  unsigned *const keys = a.keys + (size_t)wid * a.per_warp;
   for (int k = lane; k < own; k += 32) {  // the tiles that start dirty
     const int tile = wid + k * W;
     const int f = a.start ? a.start[tile] : DIRTY_FULL;
     if (ordered_sched(SCHED) && !a.start) a.prio[tile] = kUrgent;
-    if (f) atomicAdd(&words[k], f);  // (neighbours may publish already)
+    if (f) {
+      if (!ordered_sched(SCHED)) *(volatile unsigned *)&keys[k] = ~0u;  // first of all
+      atomicAdd(&words[k], f);  // (neighbours may publish already)
+    }
   }
   __syncwarp();
   for (;;) {
@@ -524,6 +532,7 @@ relax_persistent_kernel(RelaxArgs a) {
     asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];"
                  : "=l"(idle_word), "=l"(stop_word) : "l"(a.ctl) : "memory");
     const int f0 = lane < own ? *(volatile int *)&words[lane] : 0;
+    const unsigned key0 = !ordered_sched(SCHED) && lane < own ? *(volatile unsigned *)&keys[lane] : 0;
     const int thr = ordered_sched(SCHED) ? *(volatile int *)&a.ctl->thresh : 0;
     if (stop_word) break;
     int lane_wait = kClean;  // ordered: lowest priority of this lane's waiting tiles
@@ -533,7 +542,49 @@ relax_persistent_kernel(RelaxArgs a) {
       unflushed = 0;
     }
     int taken = 0;
-    for (int base = 0; base < own && taken < kTakeTiles; base += 32) {
+    if (!ordered_sched(SCHED)) {
+      // each lane's waiting tile of the lowest published value
+      unsigned best = 0;
+      int at = 0, pending = 0;
+#pragma unroll 4
+      for (int k = lane; k < own; k += 32) {
+        const int f = k == lane ? f0 : *(volatile int *)&words[k];
+        const unsigned key = (k == lane ? key0 : *(volatile unsigned *)&keys[k]) | 1u;
+        if (f && key > best) {
+          best = key;
+          at = k;
+          pending = f;
+        }
+      }
+      bool woke = false;
+      for (; taken < kTakeTiles; taken++) {
+        const unsigned top = __reduce_max_sync(0xffffffffu, best);
+        if (!top) break;
+        if (!taken) {
+          // wake: leave the idle count (before any word is taken down, below)
+          woke = idle;
+          if (idle && lane == 0) atomicAdd(&a.ctl->idle, (1ULL << 32) - 1ULL);
+          idle = false;
+        }
+        const int l = __ffs(__ballot_sync(0xffffffffu, best == top)) - 1;
+        const int k = __shfl_sync(0xffffffffu, at, l);
+        // earlier visits took time: what is pending now
+        if (taken && lane == l) pending = *(volatile int *)&words[k];
+        fence_acq_rel_gpu();  // acquire: the writes published before the word was read
+        const int got = __shfl_sync(0xffffffffu, pending, l);
+        if (lane == l) {
+          *(volatile unsigned *)&keys[k] = 0;
+          best = 0;
+        }
+        unflushed++;
+        const bool fenced = relax_tile<KIND, SCHED>(a, t, lane, wid + k * W, got);
+        if (woke && !fenced) fence_acq_rel_gpu();
+        woke = false;
+        __syncwarp();
+        if (lane == l) atomicSub(&words[k], got);  // the lane that read this word
+      }
+    }
+    for (int base = 0; ordered_sched(SCHED) && base < own && taken < kTakeTiles; base += 32) {
       const int mine = wid + (base + lane) * W;
       int f = f0;
       if (base) f = base + lane < own ? *(volatile int *)&words[base + lane] : 0;
@@ -823,7 +874,7 @@ __device__ bool relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
     // before it.
     if (__any_sync(0xffffffffu, tgt >= 0)) {
       int key = kUrgent;
-      if (ordered_sched(SCHED)) {  // the lowest changed value on the tile's edges
+      {  // the lowest changed value on the tile's edges
         float v = INFINITY;
         if ((row0 >> lane) & 1u) v = fminf(v, t.s[lane + 1][1]);
         if ((row31 >> lane) & 1u) v = fminf(v, t.s[lane + 1][kTile]);
@@ -836,8 +887,12 @@ __device__ bool relax_tile(const RelaxArgs &a, WarpTile &t, int lane, int tile, 
       __syncwarp();
       fenced = true;
       if (tgt >= 0) {
-        if (ordered_sched(SCHED)) atomicMin(&a.prio[tgt], key);
-        atomicAdd(&a.words[word_of(a, tgt, gridDim.x * kWarps)], val);
+        const int word = word_of(a, tgt, gridDim.x * kWarps);
+        if (ordered_sched(SCHED))
+          atomicMin(&a.prio[tgt], key);
+        else
+          atomicMax(&a.keys[word], ~((unsigned)key ^ 0x80000000u));
+        atomicAdd(&a.words[word], val);
       }
     }
     if (done || sweeps >= kCap) break;
@@ -1231,7 +1286,7 @@ tt_cuda_status run_queue(float *state, const float *aux, const int32_t *flats,
   if (seeded && ordered) return TT_CUDA_ERR_INVALID_ARGUMENT;  // no priorities seeded
   const int grid = relax_grid<KIND>(sched, T);
   const int W = grid * kWarps, per_warp = words_per_warp(T, W);
-  const size_t words_bytes = (size_t)W * per_warp * 4;
+  const size_t words_bytes = (size_t)W * per_warp * 8;  // and their keys
   // a fill without seeds starts everywhere and needs no flags
   const bool all = KIND == FILL && !bc;
   Workspace &ws = workspace();
@@ -1266,7 +1321,7 @@ tt_cuda_status run_queue(float *state, const float *aux, const int32_t *flats,
   if (!hctl) return TT_CUDA_ERR_ALLOC;
 
   RelaxArgs ra{state, KIND != FILL ? wcost : aux, g.m, g.n, g.tm, g.tn, ctl, dirty, words,
-               per_warp, 0, 1, prio, wmin};
+               per_warp, (unsigned *)words + (size_t)W * per_warp, 0, 1, prio, wmin};
   if (ordered) {  // no priorities, no waiting work (kClean = 0x7f7f7f7f)
     TT_CHECK(cudaMemsetAsync(prio, 0x7f, (size_t)T * 4, st));
     TT_CHECK(cudaMemsetAsync(wmin, 0x7f, (size_t)W * 4, st));
@@ -1409,7 +1464,7 @@ constexpr int kNoAllocMaxTiles = 65536;  // e.g. 8192 x 8192 pixels
 constexpr int kNoAllocMaxWarps = 8192;   // whose words are rounded up to whole sectors
 constexpr int kNoAllocHeaderWords = 64;  // control block, padded to 256 bytes
 static __device__ __align__(256) int
-    g_fill_scratch[kNoAllocHeaderWords + kNoAllocMaxTiles + kNoAllocMaxWarps * kSectorInts];
+    g_fill_scratch[kNoAllocHeaderWords + 2 * (kNoAllocMaxTiles + kNoAllocMaxWarps * kSectorInts)];
 
 namespace {
 void *g_fill_scratch_addr[64];  // device address of g_fill_scratch, per device
@@ -1449,10 +1504,10 @@ tt_cuda_status fill_noalloc(float *f, const float *dem, const uint8_t *bc,
   const int W = grid * kWarps, per_warp = words_per_warp(T, W);
   TT_LAUNCH(fill_init_kernel, elementwise_grid(g.cells()), 256, 0, st, f, dem, bc, g.m,
             g.n, nullptr, nullptr, g.tm);
-  TT_CHECK(cudaMemsetAsync(ctl, 0, (kNoAllocHeaderWords + (size_t)W * per_warp) * 4, st));
+  TT_CHECK(cudaMemsetAsync(ctl, 0, (kNoAllocHeaderWords + 2 * (size_t)W * per_warp) * 4, st));
   TT_CHECK(cudaGetLastError());
-  RelaxArgs ra{f, dem, g.m, g.n, g.tm, g.tn, ctl, nullptr, words, per_warp, 0, 1, nullptr,
-               nullptr};
+  RelaxArgs ra{f, dem, g.m, g.n, g.tm, g.tn, ctl, nullptr, words, per_warp,
+               (unsigned *)words + (size_t)W * per_warp, 0, 1, nullptr, nullptr};
   ra.max_visits = (unsigned long long)T *
                   (unsigned long long)std::min<int64_t>(max_rounds(), 1LL << 20);
   ra.visit_flush = visit_flush(ra.max_visits, W);

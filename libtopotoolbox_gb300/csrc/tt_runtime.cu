@@ -137,7 +137,7 @@ size_t CallArena::bytes(int tiles) {
   // at most (a run has no more warps than tiles, nor than fill the SMs)
   const size_t warps = std::min<size_t>(tiles, (size_t)sm_count() * 32) + 4;
   return kArenaBlocks * kBlockBytes +
-         3 * (2 * align_up((size_t)tiles * 4) + align_up(warps * 32) + 1024);
+         3 * (3 * align_up((size_t)tiles * 4) + 2 * align_up(warps * 32) + 1024);
 }
 
 tt_cuda_status CallArena::init(void *base, int tiles, cudaStream_t st) {
