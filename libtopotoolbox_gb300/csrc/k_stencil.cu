@@ -42,16 +42,18 @@ constexpr int kFp = 44;         // flat-bit column pitch (bytes): rows -1 .. 32 
                                 // conflict-free 32-bit reads (44 / 4 = 11 is odd)
 constexpr int kCountSlots = 64;
 
-// Flat test of the pixel whose 3 x 3 neighbourhood is (a0 a1 a2 | b0 b1 b2 |
-// c0 c1 c2), centre b1: not NaN and no neighbour lower, a NaN neighbour
-// counting as -INF.  A neighbour x passes when (NaN ? -INF : x) >= b1: for
-// b1 = -INF every neighbour passes, otherwise x passes exactly when
-// x >= b1 (false for NaN), one compare per neighbour.
-__device__ __forceinline__ bool is_flat(float a0, float a1, float a2, float b0, float b1,
-                                        float b2, float c0, float c1, float c2) {
-  const bool ge = (a0 >= b1) & (a1 >= b1) & (a2 >= b1) & (b0 >= b1) & (b2 >= b1) &
-                  (c0 >= b1) & (c1 >= b1) & (c2 >= b1);
-  return b1 == b1 && (ge || b1 == -INFINITY);
+// Three-input minimum that is NaN when any operand is.
+__device__ __forceinline__ float min3_nan(float a, float b, float c) {
+  float d;
+  asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// Flat test of pixel z, `lowest` the min3_nan of its 3 x 3 neighbourhood, z
+// included: not NaN and no neighbour lower, a NaN neighbour counting as -INF.
+// For z = -INF every neighbour passes; otherwise the minimum is z exactly
+// when no neighbour is lower or NaN.
+__device__ __forceinline__ bool is_flat(float lowest, float z) {
+  return (lowest == z) | (z == -INFINITY);
 }
 
 __global__ void __launch_bounds__(kBlockX * kBlockY)
@@ -110,12 +112,17 @@ identifyflats_kernel(int32_t *__restrict__ out, const float *__restrict__ dem, i
   for (int dc = 0; dc < 3; dc++)
 #pragma unroll
     for (int u = 0; u < 6; u++) z[dc][u] = zs[c + 1 + dc][r0 + 1 + u];
-  {  // flat bits of the strip, one aligned word
+  {  // flat bits of the strip, one aligned word; the rows' minima serve the
+     // three pixels above, at and below them (14 operations for four pixels
+     // instead of some 70 compares and ands, on the pipe that bounds the kernel:
+     // 16384^2 1.51 -> 1.30 ms)
     uint32_t w = 0;
+    float row[6];
+#pragma unroll
+    for (int u = 0; u < 6; u++) row[u] = min3_nan(z[0][u], z[1][u], z[2][u]);
 #pragma unroll
     for (int u = 0; u < 4; u++)
-      if (interior(r0 + u, c) && is_flat(z[0][u], z[0][u + 1], z[0][u + 2], z[1][u], z[1][u + 1],
-                                         z[1][u + 2], z[2][u], z[2][u + 1], z[2][u + 2]))
+      if (interior(r0 + u, c) && is_flat(min3_nan(row[u], row[u + 1], row[u + 2]), z[1][u + 1]))
         w |= 1u << (8 * u);
     *reinterpret_cast<uint32_t *>(&fs[c + 1][r0 + kFr]) = w;
   }
@@ -129,10 +136,10 @@ identifyflats_kernel(int32_t *__restrict__ out, const float *__restrict__ dem, i
       else if (k < 2 * (kTile + 2) + kTile) { cc = -1; rr = k - 2 * (kTile + 2); }
       else { cc = kTile; rr = k - 2 * (kTile + 2) - kTile; }
       const int zc = cc + 2, zr = rr + 2;  // staged coordinates of the pixel
-      const bool f = interior(rr, cc) &&
-                     is_flat(zs[zc - 1][zr - 1], zs[zc - 1][zr], zs[zc - 1][zr + 1],
-                             zs[zc][zr - 1], zs[zc][zr], zs[zc][zr + 1], zs[zc + 1][zr - 1],
-                             zs[zc + 1][zr], zs[zc + 1][zr + 1]);
+      const float m0 = min3_nan(zs[zc - 1][zr - 1], zs[zc - 1][zr], zs[zc - 1][zr + 1]);
+      const float m1 = min3_nan(zs[zc][zr - 1], zs[zc][zr], zs[zc][zr + 1]);
+      const float m2 = min3_nan(zs[zc + 1][zr - 1], zs[zc + 1][zr], zs[zc + 1][zr + 1]);
+      const bool f = interior(rr, cc) && is_flat(min3_nan(m0, m1, m2), zs[zc][zr]);
       fs[cc + 1][rr + kFr] = (uint8_t)f;
     }
   }
