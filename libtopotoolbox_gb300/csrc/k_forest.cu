@@ -173,9 +173,15 @@ constexpr int kRing = 4 * kTile - 4;  // 124 ring pixels
 // halves the local totals' traffic and the shared-memory atomics' width.
 template <bool U32>
 using AccT = typename std::conditional<U32, int, long long>::type;
-__device__ __forceinline__ void acc_add(int *p, int v) { atomicAdd(p, v); }
+// 64-bit addition in shared memory as two native 32-bit ones, the carry
+// handed on (a 64-bit addition there is a compare-and-swap loop; forest_up
+// 8192^2 weighted 1.26 -> 1.16 ms).  The two halves are complete once every
+// adder has been counted off.
 __device__ __forceinline__ void acc_add(long long *p, long long v) {
-  atomicAdd((unsigned long long *)p, (unsigned long long)v);
+  unsigned *const w = reinterpret_cast<unsigned *>(p);
+  const unsigned lo = (unsigned)v, hi = (unsigned)((unsigned long long)v >> 32);
+  const unsigned old = atomicAdd(w, lo);
+  atomicAdd(w + 1, hi + (old + lo < lo ? 1u : 0u));
 }
 
 // A pixel's word: its local receiver or RL_* code (16 bits), its in-tile
@@ -607,18 +613,27 @@ __global__ void coarse_link_kernel(const int *__restrict__ elist,
   }
 }
 
-// Lists the exits without coarse donors and packs every exit's coarse
-// in-degree into the high half of its link's hop count (hops <= 1025).
+// Lists the exits without coarse donors.
 __global__ void coarse_leaves_kernel(const int *__restrict__ ecount,
                                      const CoarseCell *__restrict__ ccell,
-                                     int2 *__restrict__ link, int *__restrict__ leaves,
-                                     int *__restrict__ lcount) {
+                                     int *__restrict__ leaves, int *__restrict__ lcount) {
   const int E = *ecount;
-  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < E; a += gridDim.x * blockDim.x) {
-    const int pend = ccell[a].pend;
-    link[a].y |= pend << 16;
-    if (pend == 0) leaves[append_slot(lcount)] = a;
-  }
+  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < E; a += gridDim.x * blockDim.x)
+    if (ccell[a].pend == 0) leaves[append_slot(lcount)] = a;
+}
+
+// Relaxed 128-bit load, as one access.
+__device__ __forceinline__ longlong2 load128(const CoarseCell *p) {
+  long long lo, hi;
+  asm volatile(
+      "{\n\t.reg .b128 d;\n\tld.relaxed.gpu.global.b128 d, [%2];\n\tmov.b128 {%0, %1}, d;\n\t}"
+      : "=l"(lo), "=l"(hi)
+      : "l"(p)
+      : "memory");
+  return make_longlong2(lo, hi);
+}
+__device__ __forceinline__ int cell_pending(long long hi) {
+  return (int)((unsigned long long)hi >> 32);
 }
 
 // Relaxed 128-bit compare-and-swap: (lo, hi) holds the expected value on
@@ -636,12 +651,15 @@ __device__ __forceinline__ void cas128(CoarseCell *p, unsigned long long &lo,
 
 // Last-arriver walk over the exits: a walker owns a complete exit, folds its
 // totals into the next exit downstream with one compare-and-swap, and
-// continues only if it was the last donor to arrive.  Into an exit with a
-// single coarse donor the walker is the only arrival, so it combines and
-// stores without the swap.  The longest chain of hops bounds the walk, so
-// the link and cell of the exit after the next are read while this hop's
-// swap is under way (a cell that changes meanwhile only makes its swap
-// fail and return the new value): one dependent access a hop.
+// continues only if it was the last donor to arrive.  When the cell it read
+// waits for one donor only, that is this walker, no other writes the cell any
+// more, and it combines and stores without the swap: along a river, whose
+// tributaries have mostly arrived before, most hops.  The longest chain of
+// hops bounds the walk, so the link and cell of the exit after the next are
+// read while this hop is under way (a cell that changes meanwhile only makes
+// its swap fail and return the new value): one dependent load a hop
+// (512^2 41 -> 39 us, 4096^2 171 -> 132 us, 16384^2 1.07 -> 0.98 ms; an exit
+// more read ahead, by links that name two, gained nothing).
 __global__ void coarse_walk_kernel(const int *__restrict__ leaves,
                                    const int *__restrict__ lcount,
                                    const int2 *__restrict__ link,
@@ -651,13 +669,13 @@ __global__ void coarse_walk_kernel(const int *__restrict__ leaves,
   for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < L; a += gridDim.x * blockDim.x) {
     const int e0 = leaves[a];
     // A leaf has no coarse donors: its cell was completed by earlier kernels.
-    const longlong2 c0 = __ldcg(reinterpret_cast<const longlong2 *>(&ccell[e0]));
+    const longlong2 c0 = load128(&ccell[e0]);
     long long v = c0.x;
     int hv = (int)(unsigned)(unsigned long long)c0.y;
     int2 l = link[e0];
     n_done++;
     if (l.x < 0) continue;
-    longlong2 g = __ldcg(reinterpret_cast<const longlong2 *>(&ccell[l.x]));
+    longlong2 g = load128(&ccell[l.x]);
     int2 ln = link[l.x];
     for (int guard = 0; guard < limit; guard++) {
       const int nx = l.x;
@@ -666,31 +684,29 @@ __global__ void coarse_walk_kernel(const int *__restrict__ leaves,
       longlong2 g2 = {};
       int2 l2 = {};
       if (n2 >= 0) {
-        g2 = __ldcg(reinterpret_cast<const longlong2 *>(&ccell[n2]));
+        g2 = load128(&ccell[n2]);
         l2 = link[n2];
       }
-      const int hops = l.y & 0xffff;
-      if ((ln.y >> 16) == 1) {  // the only coarse donor of nx: no other writer
-        v += g.x;
-        hv = max((int)(unsigned)(unsigned long long)g.y, hv + hops);
-        __stcg(reinterpret_cast<longlong2 *>(&ccell[nx]),
-               make_longlong2(v, (long long)(unsigned long long)(unsigned)hv));
-      } else {
-        unsigned long long lo = (unsigned long long)g.x, hi = (unsigned long long)g.y;
-        unsigned long long nlo, nhi;
-        for (;;) {
-          const int oh = (int)(unsigned)hi, op = (int)(unsigned)(hi >> 32);
-          nlo = lo + (unsigned long long)v;
-          nhi = (unsigned long long)(unsigned)max(oh, hv + hops) |
-                ((unsigned long long)(unsigned)(op - 1) << 32);
-          const unsigned long long elo = lo, ehi = hi;
-          cas128(&ccell[nx], lo, hi, nlo, nhi);
-          if (lo == elo && hi == ehi) break;  // swapped
+      const int hops = l.y;
+      unsigned long long lo = (unsigned long long)g.x, hi = (unsigned long long)g.y;
+      bool stored = false;
+      while (cell_pending((long long)hi) != 1) {  // other donors still to come
+        const unsigned long long elo = lo, ehi = hi;
+        const unsigned long long nlo = lo + (unsigned long long)v;
+        const unsigned long long nhi =
+            (unsigned long long)(unsigned)max((int)(unsigned)hi, hv + hops) |
+            ((unsigned long long)(unsigned)(cell_pending((long long)hi) - 1) << 32);
+        cas128(&ccell[nx], lo, hi, nlo, nhi);
+        if (lo == elo && hi == ehi) {
+          stored = true;
+          break;
         }
-        if ((int)(unsigned)(hi >> 32) != 1) break;  // other donors still to come
-        v = (long long)nlo;  // every donor of nx has arrived: its totals are final
-        hv = (int)(unsigned)nhi;
       }
+      if (stored) break;  // not the last donor
+      v += (long long)lo;
+      hv = max((int)(unsigned)hi, hv + hops);
+      __stcg(reinterpret_cast<longlong2 *>(&ccell[nx]),
+             make_longlong2(v, (long long)(unsigned long long)(unsigned)hv));
       n_done++;
       if (n2 < 0) break;
       l = ln;
@@ -1261,7 +1277,7 @@ tt_cuda_status up_run(const uint8_t *dir, const float *weights, int wshift,
   const int lg = list_grid(g.cells() / 8 + 1);
   TT_LAUNCH(coarse_link_kernel, lg, 256, 0, st, w.elist, w.counters + 0, dir,
             g.m, order, w.xmap, w.xsteps, w.link, w.ccell);
-  TT_LAUNCH(coarse_leaves_kernel, lg, 256, 0, st, w.counters + 0, w.ccell, w.link, w.leaves,
+  TT_LAUNCH(coarse_leaves_kernel, lg, 256, 0, st, w.counters + 0, w.ccell, w.leaves,
             w.counters + 1);
   // One walker per leaf (blocks beyond the leaf count exit at once): the
   // block scheduler hands freed SMs the next leaves, instead of each thread
