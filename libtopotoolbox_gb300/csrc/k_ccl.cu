@@ -393,12 +393,15 @@ __global__ void ccl_root_kernel(int *__restrict__ L, const LocalRoot *__restrict
   }
 }
 
-// Four pixels per thread: each level of the dependent gather (a pixel's
+// Two pixels per thread: each level of the dependent gather (a pixel's
 // local root, its global root, the root's maximum and argmax) is issued for
-// all four before any result is used.  Labels are read at flat pixels only
+// both before any result is used.  16384^2 takes 1.52 ms so, 1.65 with four
+// and 1.93 with one; 4096^2 112, 129 and 135 us.  Tiles instead of runs of
+// pixels (2.04 ms), 16-byte vectors of four (1.57) and roots that carry their
+// component's maximum, one level less (1.96 + 0.10), were slower.  Labels are read at flat pixels only
 // (the labelling writes none elsewhere); `conncomps` may be null (the
 // pipeline needs the costs alone).
-constexpr int kCostPer = 4;
+constexpr int kCostPer = 2;
 
 template <bool SEED>
 __global__ void costs_kernel(float *__restrict__ costs,
