@@ -1161,6 +1161,7 @@ struct UpWork {
   bool in_arena;  // counters: a cleared status block of the pipeline call
   int *plan;      // [0..2] deferred weighted sums' {passes, k1, d}, [4..5] their range,
                   // [8] the maximum height, kept from the pass that computed it
+  const int *hmax;  // where the node order reads the maximum height
 };
 
 // Later passes of a multi-scale sum reset the counters, so the maximum
@@ -1168,6 +1169,7 @@ struct UpWork {
 // computes the heights.
 tt_cuda_status keep_hmax(UpWork &w, cudaStream_t st) {
   TT_CHECK(cudaMemcpyAsync(w.plan + 8, w.counters + 3, sizeof(int), cudaMemcpyDeviceToDevice, st));
+  w.hmax = w.plan + 8;
   return TT_CUDA_SUCCESS;
 }
 
@@ -1189,6 +1191,7 @@ tt_cuda_status up_alloc(const GridDims &g, bool want_acc, bool want_h,
   w.in_arena = block != nullptr;
   w.counters = block ? block : (int *)ws.take(256);
   w.plan = (int *)ws.take(256);
+  w.hmax = w.counters + 3;
   w.cell = (CoarseCell *)ws.take(N * sizeof(CoarseCell));
   w.ccell = (CoarseCell *)ws.take(E * sizeof(CoarseCell));
   w.link = (int2 *)ws.take(E * 8);
@@ -1426,7 +1429,6 @@ tt_cuda_status accumulate_planned(float *acc, const uint8_t *dir, const float *w
                                   UpWork &w, cudaStream_t st, int h6[6]) {
   if (plan.passes == 1) {
     TT_TRY_STATUS(up_run(dir, weights, plan.k1, g, 0, true, want_h, acc, w, st));
-    if (want_h) TT_TRY_STATUS(keep_hmax(w, st));
     return up_status(w, st, h6);
   }
   const int64_t N = g.cells();
@@ -1484,7 +1486,7 @@ tt_cuda_status accumulate_deferred(float *acc, const uint8_t *dir, const float *
 tt_cuda_status node_scatter(ptrdiff_t *node, UpWork &w, const GridDims &g, cudaStream_t st) {
   // hist, off and cursor reuse the coarse arrays (N ints each, no longer needed).
   int *hist = w.xmap, *off = w.xsteps, *cursor = reinterpret_cast<int *>(w.cell);
-  const int *hmax = w.plan + 8;
+  const int *hmax = w.hmax;
   const int64_t N = g.cells();
   const int eg = list_grid(N);
   TT_LAUNCH(clear_bins_kernel, eg, 256, 0, st, hist, cursor, hmax, N);
@@ -1518,7 +1520,6 @@ tt_cuda_status node_order_dev(ptrdiff_t *node, const uint8_t *dir,
   UpWork w;
   TT_TRY_STATUS(up_alloc(g, false, true, w, 0, true));
   TT_TRY_STATUS(up_run(dir, nullptr, 0, g, order, false, true, nullptr, w, st));
-  TT_TRY_STATUS(keep_hmax(w, st));
   int h6[6];
   tt_cuda_status s = up_status(w, st, h6);
   if (s == TT_CUDA_ERR_CYCLE) return s;
