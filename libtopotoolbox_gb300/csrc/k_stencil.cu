@@ -1,9 +1,9 @@
 // 3x3 stencil kernels: flat/sill/presill labelling, D8 carve directions,
 // second-order gradients, hillshade and the hillshade adjoint.
 //
-// Every kernel is HBM-bound.  Tiles of 32 x 32 pixels (plus a halo) are
-// staged in shared memory with coalesced 128-byte column segments, so each
-// input byte is read from DRAM about once.
+// Each input byte is read from DRAM about once: labelling and directions walk
+// along the columns with their window in registers, the gradients' kernels
+// read tiles of 32 x 32 pixels and a halo.
 #include <algorithm>
 #include <cmath>
 
@@ -218,148 +218,200 @@ __global__ void sum_slots_kernel(const unsigned long long *__restrict__ slots,
 // contraction changes a bit.
 // ------------------------------------------------------------------
 //
-// One 32 x 32 tile per block of 32 x 8 threads.  Staging: dem and dist with
-// a one-pixel halo (NaN off the grid) and the centre flat bits.  Compute:
-// thread (tx, ty) takes column tx, rows 4 ty .. 4 ty + 3, reading the 3 x 6
-// neighbourhood of its strip once into registers.  The neighbour order is a
-// template parameter, so every offset is a compile-time constant; the IEEE
-// division of a diagonal difference by sqrt(2) runs only when the
-// difference itself beats the best slope so far (fl(diff / sqrt(2)) <= diff,
-// so otherwise it cannot win).
-// The direction bytes go out through shared memory in coalesced rows.
-// Directions of a 4-pixel column strip from its 3 x 6 window (dem z,
-// auxiliary topography d), one byte per pixel.  FLATS: whether the strip
-// may hold flats (bit 8u of fl4: pixel u is flat and compares d).
-template <unsigned ORDER, bool FLATS>
-__device__ __forceinline__ uint32_t strip_directions(const float (&z)[3][6],
-                                                     const float (&d)[3][6], uint32_t fl4,
-                                                     float sq2) {
-  uint32_t out4 = 0;
-#pragma unroll
-  for (int u = 0; u < 4; u++) {
-    const bool fl = FLATS && ((fl4 >> (8 * u)) & 1u);
-    const float zc = z[1][u + 1];
-    const float zz0 = fl ? d[1][u + 1] : zc;
-    float best = 0.0f;
-    unsigned dv = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      constexpr unsigned A = ORDER ? kD8B : kD8A, B = ORDER ? kD8A : kD8B;
-      const int di = (int)((A >> (2 * k)) & 3u) - 1, dj = (int)((B >> (2 * k)) & 3u) - 1;
-      const float zn = z[1 + dj][u + 1 + di];
-      const float zz = fl ? d[1 + dj][u + 1 + di] : zn;
-      const float diff = __fsub_rn(zz0, zz);
-      // skip higher neighbours; a difference that does not beat the best
-      // (or is NaN) cannot win, since a diagonal's quotient is <= diff
-      if (zn > zc || !(diff > best)) continue;
-      const float g = (k & 1) ? __fdiv_rn(diff, sq2) : diff;
-      if (g > best) {
-        best = g;
-        dv = 1u << k;
-      }
-    }
-    out4 |= dv << (8 * u);
-  }
-  return out4;
-}
+// The first largest slope is found without a branch per neighbour.  The
+// quotient fl(d / sqrt(2)) does not decrease with d, so the largest diagonal
+// difference has the largest diagonal quotient: one quotient a pixel instead
+// of one for each diagonal that beats the best so far.  Another diagonal has
+// the same quotient only if its difference is equal or the float before (two
+// floats further the exact quotients lie 1.4 units of the last place apart).
+// The direction is the first neighbour in order that reaches the largest
+// slope.  Quotients are a reciprocal product with an exact remainder; a warp
+// that meets a drop below 2^-100, where that remainder would underflow, takes
+// its columns again with divisions.
+//
+// Warps walk along strips of rows as in identifyflats_kernel, dem and dist of
+// three columns in registers and the next one loaded ahead (three ahead take
+// registers that hold more warps: 1.04 ms for 0.93 at 16384^2); 13 bytes a
+// pixel.  The selects of the drops and directions bound it (ALU pipe), so the
+// drops are predicated subtractions (0.93 -> 0.86 ms).  Against a tile staged
+// in shared memory with its halo and a branch per neighbour:
+// 16384^2 1.76 -> 0.86 ms, 4096^2 111 -> 66 us, 3001 x 5003 104 -> 65 us,
+// 512^2 4.3 -> 4.1 us.
+constexpr float kSq2 = 1.41421353816986083984375f;      // sqrtf(2.0f) = 0x3FB504F3
+constexpr float kInvSq2 = 0.707106769084930419921875f;  // the float next to 1 / kSq2
 
-template <unsigned ORDER>
-__global__ void __launch_bounds__(kBlockX * kBlockY)
-directions_kernel(uint8_t *__restrict__ dir, const float *__restrict__ dem,
-                  const float *__restrict__ dist,
-                  const int32_t *__restrict__ flats, int64_t m, int64_t n) {
-  __shared__ float zs[kTile + 2][kTile + 3];
-  __shared__ float ds[kTile + 2][kTile + 3];
-  __shared__ __align__(4) uint8_t fs[kTile][kTile + 4];
-  __shared__ __align__(4) uint8_t os[kTile][kTile + 4];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int64_t i0 = (int64_t)blockIdx.x * kTile;
-  const int64_t j0 = (int64_t)blockIdx.y * kTile;
-  constexpr int kH = kTile + 2;
-  constexpr int kC = (kH + kBlockY - 1) / kBlockY;  // 5 halo columns per thread row
-  const bool inner = i0 >= 1 && j0 >= 1 && i0 + kTile + 1 <= m && j0 + kTile + 1 <= n;
-  {  // every load in flight at once
-    float va[kC][2], vb[kC][2];
-    int vf[4];
-    if (inner) {
-      const float *pd = dem + (j0 - 1) * m + (i0 - 1);
-      const float *pt = dist + (j0 - 1) * m + (i0 - 1);
+template <bool WIDE>
+__device__ __forceinline__ void flag_load(int (&f)[kFlatR], const int32_t *__restrict__ flats,
+                                          int64_t row, int64_t j, int64_t m, int64_t n,
+                                          bool rows_ok) {
 #pragma unroll
-      for (int k = 0; k < kC; k++) {
-        const int c = ty + k * kBlockY;
-        const int64_t co = (int64_t)(c < kH ? c : 0) * m;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int r = tx + h * kBlockX;
-          const int rr = r < kH ? r : 0;
-          va[k][h] = pd[co + rr];
-          vb[k][h] = pt[co + rr];
-        }
-      }
+  for (int r = 0; r < kFlatR; r++) f[r] = 0;
+  if (rows_ok && j >= 0 && j < n) {
+    const int32_t *p = flats + j * m + row;
+    if constexpr (WIDE) {
+      const int4 w = *reinterpret_cast<const int4 *>(p);
+      f[0] = w.x, f[1] = w.y, f[2] = w.z, f[3] = w.w;
     } else {
 #pragma unroll
-      for (int k = 0; k < kC; k++)
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int c = ty + k * kBlockY, r = tx + h * kBlockX;
-          const int64_t i = i0 - 1 + r, j = j0 - 1 + c;
-          va[k][h] = NAN;
-          vb[k][h] = NAN;
-          if (c < kH && r < kH && i >= 0 && i < m && j >= 0 && j < n) {
-            const int64_t p = j * m + i;
-            va[k][h] = dem[p];
-            vb[k][h] = dist[p];
-          }
-        }
+      for (int r = 0; r < kFlatR; r++)
+        if (row + r < m) f[r] = p[r];
     }
-    const bool row_ok = i0 + tx < m;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int64_t j = j0 + ty + k * kBlockY;
-      vf[k] = (row_ok && j < n) ? flats[j * m + i0 + tx] : 0;
-    }
-#pragma unroll
-    for (int k = 0; k < kC; k++)
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int c = ty + k * kBlockY, r = tx + h * kBlockX;
-        if (c < kH && r < kH) {
-          zs[c][r] = va[k][h];
-          ds[c][r] = vb[k][h];
-        }
-      }
-#pragma unroll
-    for (int k = 0; k < 4; k++) fs[ty + k * kBlockY][tx] = (uint8_t)(vf[k] & 1);
   }
-  __syncthreads();
+}
+
+// fl(d / sqrt(2)): the quotient by the reciprocal and one exact remainder
+// (Markstein 1990: with a correctly rounded reciprocal the corrected quotient
+// is correctly rounded; checked for every mantissa).  For finite d of 2^-100
+// or more, where the remainder does not underflow.
+__device__ __forceinline__ float quotient_sq2(float d) {
+  const float q = __fmul_rn(d, kInvSq2);
+  return __fmaf_rn(__fmaf_rn(-q, kSq2, d), kInvSq2, q);
+}
+
+// Drop from the centre to a neighbour: in dist for a flat centre, unless the
+// neighbour is above it; in dem otherwise (negative in that case).  As a
+// predicated subtraction: a select would go to the pipe that is the busiest.
+__device__ __forceinline__ float drop_to(float zc, float zn, float dc, float dn, unsigned flat) {
+  float e;
+  asm("{.reg .pred f, p;\n"
+      " setp.ne.u32 f, %5, 0;\n"
+      " setp.leu.and.f32 p, %2, %1, f;\n"
+      " sub.rn.f32 %0, %1, %2;\n"
+      " @p sub.rn.f32 %0, %3, %4;}"
+      : "=&f"(e)
+      : "f"(zc), "f"(zn), "f"(dc), "f"(dn), "r"(flat));
+  return e;
+}
+
+// Direction of the pixel at row r of the window's middle column (column c of
+// the window is index (first + c) % 3), in byte r of the result.  FAST: the
+// quotients by quotient_sq2, and `odd` set where they may not hold (drops
+// below 2^-100); otherwise by divisions.
+template <unsigned ORDER, bool FAST>
+__device__ __forceinline__ uint32_t pixel_direction(const float (&z)[3][kFlatR + 2],
+                                                    const float (&d)[3][kFlatR + 2], int first,
+                                                    int r, unsigned fl, bool &odd) {
+  constexpr unsigned A = ORDER ? kD8B : kD8A, B = ORDER ? kD8A : kD8B;
+  const int mid = (first + 1) % 3;
+  const float zc = z[mid][r + 1], dc = d[mid][r + 1];
+  float e[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int di = (int)((A >> (2 * k)) & 3u) - 1, dj = (int)((B >> (2 * k)) & 3u) - 1;
+    const float zn = z[(first + 1 + dj) % 3][r + 1 + di];
+    const float dn = d[(first + 1 + dj) % 3][r + 1 + di];
+    e[k] = drop_to(zc, zn, dc, dn, fl);
+  }
+  // NaN differences lose every maximum and every comparison below; the least
+  // positive float as the floor is reached by none that is not positive
+  const float least = __int_as_float(1);
+  float best = max3(max3(e[0], e[2], least), e[4], e[6]);
+  const float dmax = max3(max3(e[1], e[3], 0.0f), e[5], e[7]);
+  const int bits = __float_as_int(dmax);
+  const float before = __int_as_float(bits - 1);  // NaN for dmax = 0
+  float q, qb;
+  if (FAST) {
+    odd |= (unsigned)(bits - 1) < 0x0d800000u;
+    q = dmax == INFINITY ? dmax : quotient_sq2(dmax);
+    qb = quotient_sq2(before);
+  } else {
+    q = __fdiv_rn(dmax, kSq2);
+    qb = __fdiv_rn(before, kSq2);
+  }
+  // the least diagonal difference that reaches the largest slope (NaN: none)
+  const float reach = q >= best ? (qb == q ? before : dmax) : NAN;
+  best = fmaxf(best, q);
+  uint32_t dv = 0;
+#pragma unroll
+  for (int k = 7; k >= 0; k--)
+    if ((k & 1) ? e[k] >= reach : e[k] == best) dv = 1u << (k + 8 * r);
+  return dv;
+}
+
+template <unsigned ORDER, bool FAST>
+__device__ __forceinline__ uint32_t column_directions(const float (&z)[3][kFlatR + 2],
+                                                      const float (&d)[3][kFlatR + 2],
+                                                      int first, unsigned flat, bool &odd) {
+  uint32_t o = 0;
+#pragma unroll
+  for (int r = 0; r < kFlatR; r++)
+    o |= pixel_direction<ORDER, FAST>(z, d, first, r, flat & (1u << r), odd);
+  return o;
+}
+
+// Directions of columns jb .. je - 1 of the strip whose rows start at `row` in
+// this lane.  Returns whether a quotient of this lane may not hold.
+template <unsigned ORDER, bool WIDE, bool FAST>
+__device__ __forceinline__ bool walk_directions(uint8_t *__restrict__ dir,
+                                                const float *__restrict__ dem,
+                                                const float *__restrict__ dist,
+                                                const int32_t *__restrict__ flats, int64_t m,
+                                                int64_t n, int64_t row, int64_t jb, int64_t je) {
+  constexpr int R = kFlatR;
+  const int lane = threadIdx.x & 31;
+  const bool rows_ok = row >= 0 && row < m;  // WIDE: m is a multiple of 4, all rows or none
+  const bool puts = rows_ok && lane >= 1 && lane < 31;
+
+  bool odd = false;
+  float nz[R], nd[R];  // the next column
+  int nf[R];
+  flat_load<WIDE>(nz, dem, row, jb - 1, m, n, rows_ok);
+  flat_load<WIDE>(nd, dist, row, jb - 1, m, n, rows_ok);
+  flag_load<WIDE>(nf, flats, row, jb - 1, m, n, rows_ok);
   // Off-grid neighbours hold NaN: their slope is NaN and never selected,
   // exactly as the reference skips them, so no bounds checks are needed.
-  const float sq2 = 1.41421353816986083984375f;  // sqrtf(2.0f) = 0x3FB504F3
-  {
-    const int c = tx, r0 = 4 * ty;  // centre (c + 1, r0 + 1 + u) in halo coordinates
-    float z[3][6], d[3][6];
+  float z[3][R + 2] = {}, d[3][R + 2] = {};
+  unsigned f[3] = {};
+  for (int64_t j0 = jb - 1; j0 < je + 1; j0 += 3) {
 #pragma unroll
-    for (int dc = 0; dc < 3; dc++)
+    for (int b = 0; b < 3; b++) {
+      const int64_t j = j0 + b;  // this column enters the window at index b
 #pragma unroll
-      for (int u = 0; u < 6; u++) {
-        z[dc][u] = zs[c + dc][r0 + u];
-        d[dc][u] = ds[c + dc][r0 + u];
+      for (int r = 0; r < R; r++) z[b][r + 1] = nz[r], d[b][r + 1] = nd[r];
+      f[b] = 0;
+#pragma unroll
+      for (int r = 0; r < R; r++) f[b] |= (unsigned)(nf[r] & 1) << r;
+      if (j < je) {
+        flat_load<WIDE>(nz, dem, row, j + 1, m, n, rows_ok);
+        flat_load<WIDE>(nd, dist, row, j + 1, m, n, rows_ok);
+        flag_load<WIDE>(nf, flats, row, j + 1, m, n, rows_ok);
       }
-    const uint32_t fl4 = *reinterpret_cast<const uint32_t *>(&fs[c][r0]);
-    // One code path for every strip: a second one without the flat selects
-    // measured slower (warps whose strips differ run both).
-    const uint32_t out4 = strip_directions<ORDER, true>(z, d, fl4, sq2);
-    *reinterpret_cast<uint32_t *>(&os[c][r0]) = out4;
-  }
-  __syncthreads();
-  const int64_t i = i0 + tx;
-  if (i < m)
+      z[b][0] = __shfl_up_sync(0xffffffffu, z[b][R], 1);
+      d[b][0] = __shfl_up_sync(0xffffffffu, d[b][R], 1);
+      z[b][R + 1] = __shfl_down_sync(0xffffffffu, z[b][1], 1);
+      d[b][R + 1] = __shfl_down_sync(0xffffffffu, d[b][1], 1);
+      if (j - 1 >= jb && j - 1 < je) {  // directions of column j - 1
+        const unsigned fm = f[(b + 2) % 3];
+        const uint32_t o = column_directions<ORDER, FAST>(z, d, (b + 1) % 3, fm, odd);
+        if (puts) {
+          uint8_t *p = dir + (j - 1) * m + row;
+          if constexpr (WIDE) {
+            *reinterpret_cast<uint32_t *>(p) = o;
+          } else {
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int c = ty + k * kBlockY;
-      const int64_t j = j0 + c;
-      if (j < n) dir[j * m + i] = os[c][tx];
+            for (int r = 0; r < R; r++)
+              if (row + r < m) p[r] = (uint8_t)(o >> (8 * r));
+          }
+        }
+      }
     }
+  }
+  return odd;
+}
+
+template <unsigned ORDER, bool WIDE>
+__global__ void __launch_bounds__(kFlatWarps * 32)
+directions_kernel(uint8_t *__restrict__ dir, const float *__restrict__ dem,
+                  const float *__restrict__ dist, const int32_t *__restrict__ flats, int64_t m,
+                  int64_t n, int strips, int cols) {
+  const int64_t w = (int64_t)blockIdx.x * kFlatWarps + (threadIdx.x >> 5);
+  const int64_t jb = w / strips * cols;  // first column put out
+  if (jb >= n) return;
+  const int64_t row = w % strips * kFlatRows + (int64_t)((int)(threadIdx.x & 31) - 1) * kFlatR;
+  const int64_t je = min(n, jb + cols);
+  const bool odd = walk_directions<ORDER, WIDE, true>(dir, dem, dist, flats, m, n, row, jb, je);
+  if (__any_sync(0xffffffffu, odd))  // rare: the same walk with divisions
+    walk_directions<ORDER, WIDE, false>(dir, dem, dist, flats, m, n, row, jb, je);
 }
 
 // ------------------------------------------------------------------
@@ -731,6 +783,25 @@ hillshade_bwd_kernel(float *__restrict__ gdem, const float *__restrict__ dem,
   }
 }
 
+// Strips of rows, columns per warp and blocks of a strip walk.  64 columns a
+// warp (a few more are loaded as halo), fewer until the chip has `warps_per_sm`
+// warps per SM, not below `least`.  Flats: 24 warps per SM and 4 columns (12
+// and 48 within 5 %; 8 columns at least cost 512^2 0.2 us, 2 cost 0.5).
+// Directions, more work a column: 36 warps (4096^2 66 us, 70 with 24) and 2
+// columns (512^2 4.1 us, 4.4 with 4 and 5.7 with 8).
+struct StripSplit {
+  int strips, cols;
+  unsigned blocks;
+};
+StripSplit strip_split(const GridDims &g, int warps_per_sm, int least) {
+  StripSplit s{(int)((g.m + kFlatRows - 1) / kFlatRows), 64, 0};
+  const int64_t want = (int64_t)sm_count() * warps_per_sm;
+  while (s.cols > least && s.strips * ((g.n + s.cols - 1) / s.cols) < want) s.cols /= 2;
+  const int64_t warps = s.strips * ((g.n + s.cols - 1) / s.cols);
+  s.blocks = (unsigned)((warps + kFlatWarps - 1) / kFlatWarps);
+  return s;
+}
+
 dim3 tile_grid(const GridDims &g) { return dim3(g.tm, g.tn); }
 
 }  // namespace
@@ -748,14 +819,7 @@ tt_cuda_status identifyflats_dev(int32_t *flags, const float *dem,
   }
   // Wide accesses where every column of both arrays starts on a 16-byte boundary.
   const bool wide = g.m % 4 == 0 && (((uintptr_t)flags | (uintptr_t)dem) & 15) == 0;
-  const int strips = (int)((g.m + kFlatRows - 1) / kFlatRows);
-  // Columns per warp: 64 (four more are loaded as halo), fewer until the
-  // chip has two dozen warps per SM, not below 8 (a dozen and four dozen
-  // measured the same within 5 %).
-  int cols = 64;
-  while (cols > 8 && strips * ((g.n + cols - 1) / cols) < (int64_t)sm_count() * 24) cols /= 2;
-  const int64_t warps = strips * ((g.n + cols - 1) / cols);
-  const unsigned blocks = (unsigned)((warps + kFlatWarps - 1) / kFlatWarps);
+  const auto [strips, cols, blocks] = strip_split(g, 24, 4);
   if (wide)
     TT_LAUNCH(identifyflats_kernel<true>, blocks, kFlatWarps * 32, 0, st, flags, dem, g.m, g.n,
               strips, cols, slots);
@@ -770,12 +834,14 @@ tt_cuda_status identifyflats_dev(int32_t *flags, const float *dem,
 tt_cuda_status directions_dev(uint8_t *dir, const float *dem, const float *dist,
                               const int32_t *flats, const GridDims &g,
                               unsigned order, cudaStream_t st) {
-  if (order & 1)
-    TT_LAUNCH(directions_kernel<1>, tile_grid(g), dim3(kBlockX, kBlockY), 0, st, dir, dem,
-              dist, flats, g.m, g.n);
-  else
-    TT_LAUNCH(directions_kernel<0>, tile_grid(g), dim3(kBlockX, kBlockY), 0, st, dir, dem,
-              dist, flats, g.m, g.n);
+  const bool wide =
+      g.m % 4 == 0 && (((uintptr_t)dem | (uintptr_t)dist | (uintptr_t)flats) & 15) == 0 &&
+      ((uintptr_t)dir & 3) == 0;
+  const auto [strips, cols, blocks] = strip_split(g, 36, 2);
+  const auto kernel = order & 1 ? (wide ? directions_kernel<1, true> : directions_kernel<1, false>)
+                                : (wide ? directions_kernel<0, true> : directions_kernel<0, false>);
+  TT_LAUNCH(kernel, blocks, kFlatWarps * 32, 0, st, dir, dem, dist, flats, g.m, g.n, strips,
+            cols);
   TT_CHECK(cudaGetLastError());
   return TT_CUDA_SUCCESS;
 }
