@@ -261,7 +261,7 @@ __device__ __forceinline__ void flag_load(int (&f)[kFlatR], const int32_t *__res
 
 // fl(d / sqrt(2)): the quotient by the reciprocal and one exact remainder
 // (Markstein 1990: with a correctly rounded reciprocal the corrected quotient
-// is correctly rounded; checked for every mantissa).  For finite d of 2^-100
+// is correctly rounded; checked for every float from 2^-100 up).  For finite d of 2^-100
 // or more, where the remainder does not underflow.
 __device__ __forceinline__ float quotient_sq2(float d) {
   const float q = __fmul_rn(d, kInvSq2);
