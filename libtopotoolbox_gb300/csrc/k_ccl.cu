@@ -335,8 +335,9 @@ __device__ __forceinline__ void unite_run(int *L, uint32_t a, uint32_t b, int s0
   }
 }
 
-__global__ void ccl_border_kernel(int *__restrict__ L, const uint4 *__restrict__ edges,
+__global__ void ccl_border_kernel(int *L, const uint4 *edges,
                                   int64_t m, int tm, int tn) {
+  start_after_previous();
   const int T = tm * tn;
   const int lane = threadIdx.x & 31;
   const int tile = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
@@ -381,12 +382,13 @@ __device__ __forceinline__ int root_arg(unsigned long long v) {
 // above a pixel is a local root).  The roots are final here (every union
 // is done), and a label only ever moves down to the root, so pointing a
 // local root at it while other threads still walk through it is safe.
-__global__ void ccl_root_kernel(int *__restrict__ L, const LocalRoot *__restrict__ roots,
-                                const int *__restrict__ nroots,
-                                unsigned long long *__restrict__ best) {
+__global__ void ccl_root_kernel(int *L, const LocalRoot *roots,
+                                const int *nroots,
+                                unsigned long long *best) {
+  start_after_previous();
   const int K = *nroots;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) {
-    const int4 r = __ldg(reinterpret_cast<const int4 *>(roots + k));  // pixel, key, arg
+    const int4 r = *reinterpret_cast<const int4 *>(roots + k);  // pixel, key, arg
     const int R = uf_find(L, r.x);
     if (r.y != INT_MIN) atomicMax(&best[R], pack_root(r.y, r.z));
     atomicMin(&L[r.x], R);
@@ -404,13 +406,14 @@ __global__ void ccl_root_kernel(int *__restrict__ L, const LocalRoot *__restrict
 constexpr int kCostPer = 2;
 
 template <bool SEED>
-__global__ void costs_kernel(float *__restrict__ costs,
-                             ptrdiff_t *__restrict__ conncomps, int *__restrict__ L,
-                             const unsigned long long *__restrict__ best,
-                             const int32_t *__restrict__ flats,
-                             const float *__restrict__ orig,
-                             const float *__restrict__ filled, int64_t N,
+__global__ void costs_kernel(float *costs,
+                             ptrdiff_t *conncomps, int *L,
+                             const unsigned long long *best,
+                             const int32_t *flats,
+                             const float *orig,
+                             const float *filled, int64_t N,
                              GwdtSeed seed, int64_t m, int64_t n, int tm) {
+  start_after_previous();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p0 < N;
        p0 += kCostPer * stride) {
@@ -495,14 +498,14 @@ tt_cuda_status costs_dev(float *costs, ptrdiff_t *conncomps,
   // takes longer (many runs, many unions)
   TT_LAUNCH(ccl_tile_kernel, T, kCclThreads, 0, st, L, best, roots, nroots, edges, flats, orig,
             filled, g.m, g.n, g.tm);
-  TT_LAUNCH(ccl_border_kernel, (T + 7) / 8, 256, 0, st, L, edges, g.m, g.tm, g.tn);
-  TT_LAUNCH(ccl_root_kernel, grid, 256, 0, st, L, roots, nroots, best);
+  TT_LAUNCH_NEXT(ccl_border_kernel, (T + 7) / 8, 256, 0, st, L, edges, g.m, g.tm, g.tn);
+  TT_LAUNCH_NEXT(ccl_root_kernel, grid, 256, 0, st, L, roots, nroots, best);
   const int cgrid = (int)std::min<int64_t>((N + 1023) / 1024, (int64_t)sm_count() * 32);
   if (seed)
-    TT_LAUNCH(costs_kernel<true>, cgrid, 256, 0, st, costs, conncomps, L, best,
+    TT_LAUNCH_NEXT(costs_kernel<true>, cgrid, 256, 0, st, costs, conncomps, L, best,
               flats, orig, filled, N, *seed, g.m, g.n, g.tm);
   else
-    TT_LAUNCH(costs_kernel<false>, cgrid, 256, 0, st, costs, conncomps, L, best,
+    TT_LAUNCH_NEXT(costs_kernel<false>, cgrid, 256, 0, st, costs, conncomps, L, best,
               flats, orig, filled, N, GwdtSeed{nullptr, nullptr}, g.m, g.n, g.tm);
   TT_CHECK(cudaGetLastError());
   return TT_CUDA_SUCCESS;

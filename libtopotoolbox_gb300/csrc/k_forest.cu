@@ -238,7 +238,7 @@ __device__ __forceinline__ int tile_receiver(unsigned d, int ii, int jj, bool in
 }
 
 // Stages the tile's directions with a one-pixel halo (0 off the grid).
-__device__ __forceinline__ void stage_dirs(uint8_t (*dir)[36], const uint8_t *__restrict__ g,
+__device__ __forceinline__ void stage_dirs(uint8_t (*dir)[36], const uint8_t *g,
                                            int64_t i0, int64_t j0, int64_t m, int64_t n,
                                            bool inner, int tid) {
   constexpr int kL = (kHalo * kHalo + kUpThreads - 1) / kUpThreads;
@@ -297,6 +297,7 @@ __device__ __forceinline__ int block_slots(int n, int *counter, int *sums) {
 
 template <bool ACC, bool H, unsigned ORDER, bool U32>
 __global__ void __launch_bounds__(kUpThreads, kUpBlocks) forest_up_kernel(UpArgs a) {
+  start_after_previous();
   constexpr bool COUNT = ACC && U32, SUM = ACC && !U32;
   __shared__ UpTile<SUM> t;
   const int tid = threadIdx.x;
@@ -484,6 +485,7 @@ struct FinTile {
 
 template <bool ACC, bool H, unsigned ORDER, bool U32>
 __global__ void __launch_bounds__(kUpThreads, kFinBlocks) forest_fin_kernel(UpArgs a) {
+  start_after_previous();
   using AT = AccT<U32>;
   __shared__ FinTile<U32> t;
   const int tid = threadIdx.x;
@@ -597,13 +599,14 @@ __device__ __forceinline__ int64_t receiver_of(const uint8_t *dir, int64_t p,
 
 // Coarse links, over exit ids: link(e) = {next exit, hops}, the exit
 // reached in-tile from receiver(e) and 1 + the steps to it.
-__global__ void coarse_link_kernel(const int *__restrict__ elist,
-                                   const int *__restrict__ ecount,
-                                   const uint8_t *__restrict__ dir, int64_t m,
-                                   unsigned order, const int *__restrict__ xmap,
-                                   const int *__restrict__ xsteps,
-                                   int2 *__restrict__ link,
-                                   CoarseCell *__restrict__ ccell) {
+__global__ void coarse_link_kernel(const int *elist,
+                                   const int *ecount,
+                                   const uint8_t *dir, int64_t m,
+                                   unsigned order, const int *xmap,
+                                   const int *xsteps,
+                                   int2 *link,
+                                   CoarseCell *ccell) {
+  start_after_previous();
   const int E = *ecount;
   for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < E; a += gridDim.x * blockDim.x) {
     const int64_t r = receiver_of(dir, elist[a], m, order);
@@ -614,9 +617,10 @@ __global__ void coarse_link_kernel(const int *__restrict__ elist,
 }
 
 // Lists the exits without coarse donors.
-__global__ void coarse_leaves_kernel(const int *__restrict__ ecount,
-                                     const CoarseCell *__restrict__ ccell,
-                                     int *__restrict__ leaves, int *__restrict__ lcount) {
+__global__ void coarse_leaves_kernel(const int *ecount,
+                                     const CoarseCell *ccell,
+                                     int *leaves, int *lcount) {
+  start_after_previous();
   const int E = *ecount;
   for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < E; a += gridDim.x * blockDim.x)
     if (ccell[a].pend == 0) leaves[append_slot(lcount)] = a;
@@ -660,10 +664,11 @@ __device__ __forceinline__ void cas128(CoarseCell *p, unsigned long long &lo,
 // its swap fail and return the new value): one dependent load a hop
 // (512^2 41 -> 39 us, 4096^2 171 -> 132 us, 16384^2 1.07 -> 0.98 ms; an exit
 // more read ahead, by links that name two, gained nothing).
-__global__ void coarse_walk_kernel(const int *__restrict__ leaves,
-                                   const int *__restrict__ lcount,
-                                   const int2 *__restrict__ link,
+__global__ void coarse_walk_kernel(const int *leaves,
+                                   const int *lcount,
+                                   const int2 *link,
                                    CoarseCell *ccell, int *processed, int limit) {
+  start_after_previous();
   const int L = *lcount;
   int n_done = 0;  // exits this thread completed, over all its leaves
   for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < L; a += gridDim.x * blockDim.x) {
@@ -720,10 +725,11 @@ __global__ void coarse_walk_kernel(const int *__restrict__ leaves,
 }
 
 // Final exit totals back to pixel-indexed cells for the final tile pass.
-__global__ void coarse_scatter_kernel(const int *__restrict__ ecount,
-                                      const int *__restrict__ elist,
-                                      const CoarseCell *__restrict__ ccell,
-                                      CoarseCell *__restrict__ cell) {
+__global__ void coarse_scatter_kernel(const int *ecount,
+                                      const int *elist,
+                                      const CoarseCell *ccell,
+                                      CoarseCell *cell) {
+  start_after_previous();
   const int E = *ecount;
   for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < E; a += gridDim.x * blockDim.x)
     cell[elist[a]] = ccell[a];
@@ -742,8 +748,9 @@ __device__ __forceinline__ int height_bins(const int *hmax, int64_t N) {
   return (int)(H < N ? (H > 0 ? H : 0) : N);
 }
 
-__global__ void clear_bins_kernel(int *__restrict__ hist, int *__restrict__ cursor,
-                                  const int *__restrict__ hmax, int64_t N) {
+__global__ void clear_bins_kernel(int *hist, int *cursor,
+                                  const int *hmax, int64_t N) {
+  start_after_previous();
   const int H = height_bins(hmax, N);
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < H; b += gridDim.x * blockDim.x) {
     hist[b] = 0;
@@ -751,8 +758,9 @@ __global__ void clear_bins_kernel(int *__restrict__ hist, int *__restrict__ curs
   }
 }
 
-__global__ void h_hist_kernel(const int *__restrict__ h, int64_t N,
-                              int *__restrict__ hist, const int *__restrict__ hmax) {
+__global__ void h_hist_kernel(const int *h, int64_t N,
+                              int *hist, const int *hmax) {
+  start_after_previous();
   __shared__ int sb[kSmallBins];
   const int H = height_bins(hmax, N);
   for (int b = threadIdx.x; b < kSmallBins; b += blockDim.x) sb[b] = 0;
@@ -775,9 +783,10 @@ __global__ void h_hist_kernel(const int *__restrict__ h, int64_t N,
 }
 
 // Exclusive scan of the height bins by one block of 1024 threads.
-__global__ void __launch_bounds__(1024) scan_kernel(const int *__restrict__ in,
-                                                    int *__restrict__ out,
-                                                    const int *__restrict__ hmax, int64_t N) {
+__global__ void __launch_bounds__(1024) scan_kernel(const int *in,
+                                                    int *out,
+                                                    const int *hmax, int64_t N) {
+  start_after_previous();
   __shared__ int part[1024];
   const int tid = threadIdx.x;
   const int n = height_bins(hmax, N);
@@ -803,11 +812,12 @@ __global__ void __launch_bounds__(1024) scan_kernel(const int *__restrict__ in,
 
 constexpr int kScatterPer = 8;  // elements per thread per chunk
 
-__global__ void node_scatter_kernel(const int *__restrict__ h, int64_t N,
-                                    const int *__restrict__ off,
-                                    int *__restrict__ cursor,
-                                    ptrdiff_t *__restrict__ node,
-                                    const int *__restrict__ hmax) {
+__global__ void node_scatter_kernel(const int *h, int64_t N,
+                                    const int *off,
+                                    int *cursor,
+                                    ptrdiff_t *node,
+                                    const int *hmax) {
+  start_after_previous();
   __shared__ int cnt[kSmallBins];
   __shared__ int base[kSmallBins];
   const int H = height_bins(hmax, N);
@@ -1276,23 +1286,23 @@ tt_cuda_status up_run(const uint8_t *dir, const float *weights, int wshift,
     fin = order ? forest_fin_kernel<false, true, 1, false>
                 : forest_fin_kernel<false, true, 0, false>;
   }
-  TT_LAUNCH(up, tgrid, kUpThreads, 0, st, a);
+  TT_LAUNCH_NEXT(up, tgrid, kUpThreads, 0, st, a);
   const int lg = list_grid(g.cells() / 8 + 1);
-  TT_LAUNCH(coarse_link_kernel, lg, 256, 0, st, w.elist, w.counters + 0, dir,
+  TT_LAUNCH_NEXT(coarse_link_kernel, lg, 256, 0, st, w.elist, w.counters + 0, dir,
             g.m, order, w.xmap, w.xsteps, w.link, w.ccell);
-  TT_LAUNCH(coarse_leaves_kernel, lg, 256, 0, st, w.counters + 0, w.ccell, w.leaves,
+  TT_LAUNCH_NEXT(coarse_leaves_kernel, lg, 256, 0, st, w.counters + 0, w.ccell, w.leaves,
             w.counters + 1);
   // One walker per leaf (blocks beyond the leaf count exit at once): the
   // block scheduler hands freed SMs the next leaves, instead of each thread
   // walking a fixed share of them one after another.
   const int64_t exits = std::min<int64_t>(g.cells(), (int64_t)g.tiles() * kRing);
   const int wg = (int)std::max<int64_t>(1, std::min<int64_t>((exits + 255) / 256, INT_MAX));
-  TT_LAUNCH(coarse_walk_kernel, wg, 256, 0, st, w.leaves, w.counters + 1, w.link,
+  TT_LAUNCH_NEXT(coarse_walk_kernel, wg, 256, 0, st, w.leaves, w.counters + 1, w.link,
             w.ccell, w.counters + 2, (int)std::min<int64_t>(g.cells(), INT_MAX));
-  TT_LAUNCH(coarse_scatter_kernel, lg, 256, 0, st, w.counters + 0, w.elist, w.ccell,
+  TT_LAUNCH_NEXT(coarse_scatter_kernel, lg, 256, 0, st, w.counters + 0, w.elist, w.ccell,
             w.cell);
   a.phase = 3;
-  TT_LAUNCH(fin, fgrid, kUpThreads, 0, st, a);
+  TT_LAUNCH_NEXT(fin, fgrid, kUpThreads, 0, st, a);
   TT_CHECK(cudaGetLastError());
   return TT_CUDA_SUCCESS;
 }
@@ -1489,10 +1499,10 @@ tt_cuda_status node_scatter(ptrdiff_t *node, UpWork &w, const GridDims &g, cudaS
   const int *hmax = w.hmax;
   const int64_t N = g.cells();
   const int eg = list_grid(N);
-  TT_LAUNCH(clear_bins_kernel, eg, 256, 0, st, hist, cursor, hmax, N);
-  TT_LAUNCH(h_hist_kernel, eg, 256, 0, st, w.h, N, hist, hmax);
-  TT_LAUNCH(scan_kernel, 1, 1024, 0, st, hist, off, hmax, N);
-  TT_LAUNCH(node_scatter_kernel, eg, 256, 0, st, w.h, N, off, cursor, node, hmax);
+  TT_LAUNCH_NEXT(clear_bins_kernel, eg, 256, 0, st, hist, cursor, hmax, N);
+  TT_LAUNCH_NEXT(h_hist_kernel, eg, 256, 0, st, w.h, N, hist, hmax);
+  TT_LAUNCH_NEXT(scan_kernel, 1, 1024, 0, st, hist, off, hmax, N);
+  TT_LAUNCH_NEXT(node_scatter_kernel, eg, 256, 0, st, w.h, N, off, cursor, node, hmax);
   TT_CHECK(cudaGetLastError());
   return TT_CUDA_SUCCESS;
 }

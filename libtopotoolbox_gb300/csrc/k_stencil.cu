@@ -79,7 +79,7 @@ constexpr int kFlatR = 4;                  // rows per lane
 constexpr int kFlatRows = kFlatR * 30;     // rows a warp puts out
 
 template <bool WIDE>
-__device__ __forceinline__ void flat_load(float (&v)[kFlatR], const float *__restrict__ dem,
+__device__ __forceinline__ void flat_load(float (&v)[kFlatR], const float *dem,
                                           int64_t row, int64_t j, int64_t m, int64_t n,
                                           bool rows_ok) {
 #pragma unroll
@@ -99,8 +99,9 @@ __device__ __forceinline__ void flat_load(float (&v)[kFlatR], const float *__res
 
 template <bool WIDE>
 __global__ void __launch_bounds__(kFlatWarps * 32)
-identifyflats_kernel(int32_t *__restrict__ out, const float *__restrict__ dem, int64_t m,
+identifyflats_kernel(int32_t *out, const float *dem, int64_t m,
                      int64_t n, int strips, int cols, unsigned long long *slots) {
+  start_after_previous();
   constexpr int R = kFlatR;
   const int lane = threadIdx.x & 31;
   const int64_t w = (int64_t)blockIdx.x * kFlatWarps + (threadIdx.x >> 5);
@@ -241,7 +242,7 @@ constexpr float kSq2 = 1.41421353816986083984375f;      // sqrtf(2.0f) = 0x3FB50
 constexpr float kInvSq2 = 0.707106769084930419921875f;  // the float next to 1 / kSq2
 
 template <bool WIDE>
-__device__ __forceinline__ void flag_load(int (&f)[kFlatR], const int32_t *__restrict__ flats,
+__device__ __forceinline__ void flag_load(int (&f)[kFlatR], const int32_t *flats,
                                           int64_t row, int64_t j, int64_t m, int64_t n,
                                           bool rows_ok) {
 #pragma unroll
@@ -342,10 +343,10 @@ __device__ __forceinline__ uint32_t column_directions(const float (&z)[3][kFlatR
 // Directions of columns jb .. je - 1 of the strip whose rows start at `row` in
 // this lane.  Returns whether a quotient of this lane may not hold.
 template <unsigned ORDER, bool WIDE, bool FAST>
-__device__ __forceinline__ bool walk_directions(uint8_t *__restrict__ dir,
-                                                const float *__restrict__ dem,
-                                                const float *__restrict__ dist,
-                                                const int32_t *__restrict__ flats, int64_t m,
+__device__ __forceinline__ bool walk_directions(uint8_t *dir,
+                                                const float *dem,
+                                                const float *dist,
+                                                const int32_t *flats, int64_t m,
                                                 int64_t n, int64_t row, int64_t jb, int64_t je) {
   constexpr int R = kFlatR;
   const int lane = threadIdx.x & 31;
@@ -401,9 +402,10 @@ __device__ __forceinline__ bool walk_directions(uint8_t *__restrict__ dir,
 
 template <unsigned ORDER, bool WIDE>
 __global__ void __launch_bounds__(kFlatWarps * 32)
-directions_kernel(uint8_t *__restrict__ dir, const float *__restrict__ dem,
-                  const float *__restrict__ dist, const int32_t *__restrict__ flats, int64_t m,
+directions_kernel(uint8_t *dir, const float *dem,
+                  const float *dist, const int32_t *flats, int64_t m,
                   int64_t n, int strips, int cols) {
+  start_after_previous();
   const int64_t w = (int64_t)blockIdx.x * kFlatWarps + (threadIdx.x >> 5);
   const int64_t jb = w / strips * cols;  // first column put out
   if (jb >= n) return;
@@ -821,10 +823,10 @@ tt_cuda_status identifyflats_dev(int32_t *flags, const float *dem,
   const bool wide = g.m % 4 == 0 && (((uintptr_t)flags | (uintptr_t)dem) & 15) == 0;
   const auto [strips, cols, blocks] = strip_split(g, 24, 4);
   if (wide)
-    TT_LAUNCH(identifyflats_kernel<true>, blocks, kFlatWarps * 32, 0, st, flags, dem, g.m, g.n,
+    TT_LAUNCH_NEXT(identifyflats_kernel<true>, blocks, kFlatWarps * 32, 0, st, flags, dem, g.m, g.n,
               strips, cols, slots);
   else
-    TT_LAUNCH(identifyflats_kernel<false>, blocks, kFlatWarps * 32, 0, st, flags, dem, g.m, g.n,
+    TT_LAUNCH_NEXT(identifyflats_kernel<false>, blocks, kFlatWarps * 32, 0, st, flags, dem, g.m, g.n,
               strips, cols, slots);
   if (count_dev) TT_LAUNCH(sum_slots_kernel, 1, 32, 0, st, slots, count_dev);
   TT_CHECK(cudaGetLastError());
@@ -840,7 +842,7 @@ tt_cuda_status directions_dev(uint8_t *dir, const float *dem, const float *dist,
   const auto [strips, cols, blocks] = strip_split(g, 36, 2);
   const auto kernel = order & 1 ? (wide ? directions_kernel<1, true> : directions_kernel<1, false>)
                                 : (wide ? directions_kernel<0, true> : directions_kernel<0, false>);
-  TT_LAUNCH(kernel, blocks, kFlatWarps * 32, 0, st, dir, dem, dist, flats, g.m, g.n, strips,
+  TT_LAUNCH_NEXT(kernel, blocks, kFlatWarps * 32, 0, st, dir, dem, dist, flats, g.m, g.n, strips,
             cols);
   TT_CHECK(cudaGetLastError());
   return TT_CUDA_SUCCESS;
