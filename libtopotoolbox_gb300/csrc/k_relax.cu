@@ -1216,9 +1216,10 @@ inline bool aligned4(const void *p) { return ((uintptr_t)p & 3u) == 0; }
 
 // Smallest grid side that starts the fill from a coarse bound (0: never);
 // TT_CUDA_FILL_BOUND_MIN overrides it.  Measured on the 16384² workload
-// generator: 16384² 10.11 -> 9.45 ms (visits per tile 5 -> 3), 8192² no
-// change, 4096² slower (1.13 -> 1.42 ms: the coarse run and the full first
-// visit of every tile cost more than the visits saved).
+// generator, without and with the bound: 16384² 7.16 and 6.39 ms, 12288² 4.20
+// and 3.99, 10240² 3.27 and 3.03, 8192² 2.19 and 2.17, 4096² 0.60 and 0.85
+// (the coarse run and the full first visit of every tile cost more than the
+// visits saved).
 int64_t fill_bound_min() {
   static const int64_t v = [] {
     const char *s = std::getenv("TT_CUDA_FILL_BOUND_MIN");
