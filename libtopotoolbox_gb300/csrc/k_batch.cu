@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <cmath>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "tt_internal.cuh"
@@ -34,9 +35,7 @@ struct tt_cuda_batch {
   int64_t Mc = 0, Nc = 0;               // canvas rows (fast) and columns
   std::vector<int64_t> m, n, i0, j0;     // per DEM
   std::vector<int64_t> off;              // prefix of m*n, size count+1
-  int64_t columns = 0;                   // sum of n
-  int64_t *d_tab = nullptr;              // device: m, n, i0, j0, off and the columns' prefix
-                                         // (count each, the prefixes count + 1)
+  int64_t *d_tab = nullptr;              // device: m, n, i0, j0, off (5 x count, off count+1)
   void **d_ptr = nullptr;                // device pointer table, 7 x count
   std::vector<const void *> cap_ptr;     // pointers the graph was captured with
   float *dem = nullptr, *filled = nullptr, *costs = nullptr, *dist = nullptr, *acc = nullptr;
@@ -65,73 +64,98 @@ __device__ __forceinline__ int find_dem(const int64_t *off, int count, int64_t q
   return lo;
 }
 
-// Copies between the DEMs and the canvas go a column of one DEM per warp:
-// the DEM is looked up once a column, and both sides are contiguous along
-// it.  (A look-up, a division and a remainder for every pixel took 113 us to
-// pack and 283 us to unpack 14.6 M pixels in 64 DEMs; 33 and 131 us now.)
-struct Column {
-  int dem;
-  int64_t rows, at, canvas;  // first pixel in the DEM and in the canvas
-};
-__device__ __forceinline__ Column find_column(const int64_t *__restrict__ tab, int count,
-                                              int64_t c, int64_t Mc) {
-  const int64_t *m = tab, *i0 = tab + 2 * count, *j0 = tab + 3 * count;
-  const int64_t *coff = tab + 5 * count + 1;  // prefix of the columns
-  const int b = find_dem(coff, count, c);
-  const int64_t j = c - coff[b];
-  return Column{b, m[b], j * m[b], (j0[b] + j) * Mc + i0[b]};
+// Copies between the DEMs and the canvas go by runs of kRun pixels of the DEMs
+// laid end to end, a run per warp: the DEM is looked up and the position divided
+// into column and row once a run, and a lane goes on from there, 32 pixels at a
+// time, by additions, whatever the DEMs' shapes.  A warp per DEM column left
+// lanes idle on DEMs of fewer than 32 rows and warps on DEMs of few columns (64
+// DEMs of 1 x 8192 pixels: the batch 821 us, 322 now); a look-up, a division and
+// a remainder for every pixel took 113 us to pack and 283 us to unpack 14.6 M
+// pixels in 64 DEMs, which take 36 and 129 now.
+constexpr int kCopy = 8;           // loads of a lane in flight
+constexpr int kRun = 32 * kCopy * 2;  // (half and twice as long: the same)
+
+// Copies `n` pixels from DEM pixel l0 on, `at` their places in the canvas (-1:
+// none), lane by lane.
+template <bool PACK, class T>
+__device__ __forceinline__ void copy_run(T *dem, T *canvas, int64_t l0, const int (&at)[kCopy]) {
+  T v[kCopy];
+#pragma unroll
+  for (int u = 0; u < kCopy; u++)
+    if (at[u] >= 0) v[u] = PACK ? dem[l0 + 32 * u] : canvas[at[u]];
+#pragma unroll
+  for (int u = 0; u < kCopy; u++)
+    if (at[u] >= 0) {
+      if (PACK)
+        canvas[at[u]] = v[u];
+      else
+        dem[l0 + 32 * u] = v[u];
+    }
 }
 
-// One warp copies `n` contiguous elements, kCopy loads of a lane in flight.
-constexpr int kCopy = 8;
-template <class T>
-__device__ __forceinline__ void warp_copy(T *__restrict__ to, const T *__restrict__ from,
-                                          int64_t n, int lane) {
-  for (int64_t i0 = lane; i0 < n; i0 += 32 * kCopy) {
-    T v[kCopy];
+// Calls copy(dem, first pixel of this lane, its kCopy places in the canvas) over
+// the runs of this warp.
+template <class F>
+__device__ __forceinline__ void for_runs(const int64_t *__restrict__ tab, int count,
+                                         int64_t total, int64_t Mc, F &&copy) {
+  const int64_t *m = tab, *i0 = tab + 2 * count, *j0 = tab + 3 * count, *off = tab + 4 * count;
+  const int lane = threadIdx.x & 31;
+  const int64_t step = ((int64_t)gridDim.x * blockDim.x >> 5) * kRun;
+  for (int64_t r = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * kRun; r < total;
+       r += step) {
+    const int64_t end = min(total, r + kRun);
+    int64_t q = r;
+    for (int b = find_dem(off, count, q); q < end; b++) {
+      const int64_t first = off[b], last = min(end, off[b + 1]);
+      // (a canvas, and so a DEM, has below 2^31 pixels)
+      const unsigned rows = (unsigned)m[b], l = (unsigned)(q - first) + lane;
+      const unsigned j = l / rows, dj = 32 / rows, di = 32 - dj * rows;
+      unsigned i = l - j * rows;
+      unsigned p = (unsigned)((j0[b] + j) * Mc + i0[b] + i);
+      const unsigned dp = (unsigned)(dj * Mc + di), wrap = (unsigned)(Mc - rows);
+      for (; q < last; q += 32 * kCopy) {
+        int at[kCopy];
 #pragma unroll
-    for (int u = 0; u < kCopy; u++)
-      if (i0 + 32 * u < n) v[u] = from[i0 + 32 * u];
-#pragma unroll
-    for (int u = 0; u < kCopy; u++)
-      if (i0 + 32 * u < n) to[i0 + 32 * u] = v[u];
+        for (int u = 0; u < kCopy; u++) {
+          at[u] = q + 32 * u + lane < last ? (int)p : -1;
+          i += di;
+          p += dp;
+          if (i >= rows) {  // into the column after
+            i -= rows;
+            p += wrap;
+          }
+        }
+        copy(b, q - first + lane, at);
+      }
+      q = last;
+    }
   }
 }
 
 // canvas <- DEMs and boundary conditions
 __global__ void pack_kernel(const int64_t *__restrict__ tab, void *const *__restrict__ ptr,
-                            int count, int64_t columns, int64_t Mc, float *cdem, uint8_t *cbc) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * blockDim.x >> 5;
-  for (int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; c < columns;
-       c += warps) {
-    const Column k = find_column(tab, count, c, Mc);
-    const float *const dem = (const float *)ptr[P_DEM * count + k.dem] + k.at;
-    const uint8_t *const bc = (const uint8_t *)ptr[P_BC * count + k.dem] + k.at;
-    warp_copy(cdem + k.canvas, dem, k.rows, lane);
-    warp_copy(cbc + k.canvas, bc, k.rows, lane);
-  }
+                            int count, int64_t total, int64_t Mc, float *cdem, uint8_t *cbc) {
+  for_runs(tab, count, total, Mc, [&](int b, int64_t l0, const int (&at)[kCopy]) {
+    copy_run<true>((float *)ptr[P_DEM * count + b], cdem, l0, at);
+    copy_run<true>((uint8_t *)ptr[P_BC * count + b], cbc, l0, at);
+  });
 }
 
 // DEM outputs <- canvas (an output family with a NULL table entry is skipped)
 __global__ void unpack_kernel(const int64_t *__restrict__ tab, void *const *__restrict__ ptr,
-                              int count, int64_t columns, int64_t Mc, const float *filled,
-                              const int32_t *flats, const float *dist, const uint8_t *dir,
-                              const float *acc) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * blockDim.x >> 5;
-  for (int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; c < columns;
-       c += warps) {
-    const Column k = find_column(tab, count, c, Mc);
-    auto copy = [&](auto *to, const auto *from) {
-      if (to) warp_copy(to + k.at, from + k.canvas, k.rows, lane);
+                              int count, int64_t total, int64_t Mc, float *filled,
+                              int32_t *flats, float *dist, uint8_t *dir, float *acc) {
+  for_runs(tab, count, total, Mc, [&](int b, int64_t l0, const int (&at)[kCopy]) {
+    auto copy = [&](int family, auto *canvas) {
+      using T = std::remove_pointer_t<decltype(canvas)>;
+      if (T *to = (T *)ptr[family * count + b]) copy_run<false>(to, canvas, l0, at);
     };
-    copy((float *)ptr[P_FILLED * count + k.dem], filled);
-    copy((int32_t *)ptr[P_FLATS * count + k.dem], flats);
-    copy((float *)ptr[P_DIST * count + k.dem], dist);
-    copy((uint8_t *)ptr[P_DIR * count + k.dem], dir);
-    copy((float *)ptr[P_ACC * count + k.dem], acc);
-  }
+    copy(P_FILLED, filled);
+    copy(P_FLATS, flats);
+    copy(P_DIST, dist);
+    copy(P_DIR, dir);
+    copy(P_ACC, acc);
+  });
 }
 
 int ew_grid(int64_t N) {
@@ -171,11 +195,13 @@ tt_cuda_status enqueue(tt_cuda_batch *b, cudaStream_t st) {
   const int64_t N = b->Mc * b->Nc;
   const ptrdiff_t dims[2] = {(ptrdiff_t)b->Mc, (ptrdiff_t)b->Nc};
   const GridDims g = make_dims(dims);
+  const int64_t total = b->off[b->count];
+  const int copy_grid = ew_grid((total + kRun - 1) / kRun * 32);
   TT_CHECK(cudaMemsetAsync(b->d_sink, 0, (size_t)b->sink_cap * kRecordInts * 4, st));
   TT_CHECK(cudaMemsetAsync(b->dem, 0xff, (size_t)N * 4, st));  // NaN gutters
   TT_CHECK(cudaMemsetAsync(b->bc, 0, (size_t)N, st));
-  TT_LAUNCH(pack_kernel, ew_grid(b->columns * 32), 256, 0, st, b->d_tab, b->d_ptr, b->count,
-            b->columns, b->Mc, b->dem, b->bc);
+  TT_LAUNCH(pack_kernel, copy_grid, 256, 0, st, b->d_tab, b->d_ptr, b->count, total, b->Mc,
+            b->dem, b->bc);
   TT_CHECK(cudaGetLastError());
   tt_cuda_status s;
   if ((s = fill_dev(b->filled, b->dem, b->bc, g, st, false)) != TT_CUDA_SUCCESS) return s;
@@ -186,8 +212,8 @@ tt_cuda_status enqueue(tt_cuda_batch *b, cudaStream_t st) {
   if ((s = directions_dev(b->dir, b->filled, b->dist, b->flats, g, 0, st)) != TT_CUDA_SUCCESS)
     return s;
   if ((s = accumulate_dev(b->acc, b->dir, nullptr, g, st)) != TT_CUDA_SUCCESS) return s;
-  TT_LAUNCH(unpack_kernel, ew_grid(b->columns * 32), 256, 0, st, b->d_tab, b->d_ptr, b->count,
-            b->columns, b->Mc, b->filled, b->flats, b->dist, b->dir, b->acc);
+  TT_LAUNCH(unpack_kernel, copy_grid, 256, 0, st, b->d_tab, b->d_ptr, b->count, total, b->Mc,
+            b->filled, b->flats, b->dist, b->dir, b->acc);
   TT_CHECK(cudaGetLastError());
   return TT_CUDA_SUCCESS;
 }
@@ -265,11 +291,6 @@ tt_cuda_status tt_cuda_batch_create(int count, const ptrdiff_t *dims, int64_t ca
   std::vector<int64_t> tab;
   for (auto *v : {&b->m, &b->n, &b->i0, &b->j0}) tab.insert(tab.end(), v->begin(), v->end());
   tab.insert(tab.end(), b->off.begin(), b->off.end());
-  for (int k = 0; k < count; k++) {
-    tab.push_back(b->columns);
-    b->columns += b->n[k];
-  }
-  tab.push_back(b->columns);
   bool ok = cudaMalloc(&b->d_tab, tab.size() * 8) == cudaSuccess &&
             cudaMalloc(&b->d_ptr, (size_t)P_COUNT * count * sizeof(void *)) == cudaSuccess &&
             cudaMalloc(&b->dem, N * 4) == cudaSuccess &&
