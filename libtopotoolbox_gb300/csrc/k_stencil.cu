@@ -6,6 +6,7 @@
 // read tiles of 32 x 32 pixels and a halo.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "tt_internal.cuh"
 
@@ -32,13 +33,14 @@ constexpr int kBlockY = 8;   // along j
 // minima and maxima, NaN standing for "not of this kind".
 //
 // A warp walks along the columns of a strip of rows, four consecutive rows per
-// lane (120 of its 128 rows are put out, the outer lanes are the halo), with the last three columns in registers: a column's vertical
-// neighbours come from the lane's own rows and one shuffle each way, the
-// flat bits of the rows beside them from two ballots.  Nothing is staged in
-// shared memory, and a pixel costs some 20 operations instead of the 150 of
-// a tile staged with its halo and eight compares a pixel, which the ALU pipe
-// bounded (85 % busy): 16384^2 1.30 -> 0.45 ms (4.8 TB/s of 2.1 GB), 4096^2
-// 84 -> 36 us, 3001 x 5003 75 -> 41 us, 512^2 3.1 -> 3.6 us.
+// lane (120 of its 128 rows are put out, the outer lanes are the halo), with
+// the last three columns in registers: a column's vertical neighbours come
+// from the lane's own rows and one shuffle each way, the flat bits of the rows
+// beside them from two ballots.  Nothing is staged in shared memory, and a
+// pixel costs some 20 operations instead of the 150 of a tile staged with its
+// halo and eight compares a pixel, which the ALU pipe bounded (85 % busy):
+// 16384^2 1.30 -> 0.45 ms (4.8 TB/s of 2.1 GB), 4096^2 84 -> 37 us, 3001 x 5003
+// 75 -> 42 us, 512^2 3.1 -> 3.6 us.
 //
 // WIDE: 16-byte loads and stores, where every column starts on a 16-byte
 // boundary.  Elsewhere four strided ones, which L1 and L2 put together (one
@@ -75,8 +77,10 @@ __device__ __forceinline__ bool is_flat(float lowest, float z) {
   return (lowest == z) | (z == -INFINITY);
 }
 
-constexpr int kFlatR = 4;                  // rows per lane
-constexpr int kFlatRows = kFlatR * 30;     // rows a warp puts out
+// A strip takes `lanes` lanes, the outer two its halo, and puts out
+// (lanes - 2) * kFlatR rows: the 32 lanes of a warp along one, or NARROW along
+// several strips of `seg` lanes each, in step (see strip_split).
+constexpr int kFlatR = 4;  // rows per lane
 
 template <bool WIDE>
 __device__ __forceinline__ void flat_load(float (&v)[kFlatR], const float *dem,
@@ -97,24 +101,29 @@ __device__ __forceinline__ void flat_load(float (&v)[kFlatR], const float *dem,
   }
 }
 
-template <bool WIDE>
+template <bool WIDE, bool NARROW>
 __global__ void __launch_bounds__(kFlatWarps * 32)
 identifyflats_kernel(int32_t *out, const float *dem, int64_t m,
-                     int64_t n, int strips, int cols, unsigned long long *slots) {
+                     int64_t n, int strips, int cols, int seg, unsigned long long *slots) {
   start_after_previous();
   constexpr int R = kFlatR;
   const int lane = threadIdx.x & 31;
   const int64_t w = (int64_t)blockIdx.x * kFlatWarps + (threadIdx.x >> 5);
-  const int64_t jb = w / strips * cols;  // first column put out
-  if (jb >= n) return;
-  const int64_t row = w % strips * kFlatRows + (int64_t)(lane - 1) * R;
+  const int lanes = NARROW ? seg : 32, sl = NARROW ? lane & (seg - 1) : lane;
+  const int64_t first = NARROW ? w * (32 / seg) : w;
+  const int64_t walk = NARROW ? first + lane / seg : w;
+  const int64_t jb = walk / strips * cols;  // first column put out
+  if ((NARROW ? first / strips * cols : jb) >= n) return;
+  const int64_t row = walk % strips * ((lanes - 2) * R) + (int64_t)(sl - 1) * R;
   const bool rows_ok = row >= 0 && row < m;  // WIDE: m is a multiple of 4, all rows or none
-  const bool puts = rows_ok && lane >= 1 && lane < 31;
+  const bool puts = rows_ok && sl >= 1 && sl < lanes - 1;  // sl: lane of the strip
   const int64_t je = min(n, jb + cols);
+  const int64_t end = NARROW ? jb + cols : je;  // the strips of a warp walk in step
   bool inner_row[R];  // interior pixels may be flat
 #pragma unroll
   for (int r = 0; r < R; r++) inner_row[r] = row + r >= 1 && row + r < m - 1;
-  const uint32_t lane_up = lane ? 1u << (lane - 1) : 0u, lane_dn = lane < 31 ? 2u << lane : 0u;
+  const uint32_t lane_up = sl ? 1u << (lane - 1) : 0u;
+  const uint32_t lane_dn = sl < lanes - 1 ? 2u << lane : 0u;
 
   float next[kFlatBatch][R];
 #pragma unroll
@@ -129,21 +138,21 @@ identifyflats_kernel(int32_t *out, const float *dem, int64_t m,
   bool f2[R] = {};
   float up1 = 0.f, dn1 = 0.f;
   unsigned cnt = 0;
-  for (int64_t j0 = jb - 2; j0 < je + 2; j0 += kFlatBatch) {
+  for (int64_t j0 = jb - 2; j0 < end + 2; j0 += kFlatBatch) {
     float cur[kFlatBatch][R];
 #pragma unroll
     for (int b = 0; b < kFlatBatch; b++)
 #pragma unroll
       for (int r = 0; r < R; r++) cur[b][r] = next[b][r];
-    if (j0 + kFlatBatch < je + 2)
+    if (j0 + kFlatBatch < end + 2)
 #pragma unroll
       for (int b = 0; b < kFlatBatch; b++)
         flat_load<WIDE>(next[b], dem, row, j0 + kFlatBatch + b, m, n, rows_ok);
 #pragma unroll
     for (int b = 0; b < kFlatBatch; b++) {
       const int64_t j = j0 + b;
-      const float up0 = __shfl_up_sync(0xffffffffu, cur[b][R - 1], 1);
-      const float dn0 = __shfl_down_sync(0xffffffffu, cur[b][0], 1);
+      const float up0 = __shfl_up_sync(0xffffffffu, cur[b][R - 1], 1, lanes);
+      const float dn0 = __shfl_down_sync(0xffffffffu, cur[b][0], 1, lanes);
       // flat test of column j - 1
       float m0[R], g1[R], h1[R], G[R + 2], H[R + 2];
       bool f1[R];
@@ -340,18 +349,18 @@ __device__ __forceinline__ uint32_t column_directions(const float (&z)[3][kFlatR
   return o;
 }
 
-// Directions of columns jb .. je - 1 of the strip whose rows start at `row` in
+// Directions of columns jb .. jb + cols - 1 of the strip whose rows start at `row` in
 // this lane.  Returns whether a quotient of this lane may not hold.
-template <unsigned ORDER, bool WIDE, bool FAST>
-__device__ __forceinline__ bool walk_directions(uint8_t *dir,
-                                                const float *dem,
-                                                const float *dist,
-                                                const int32_t *flats, int64_t m,
-                                                int64_t n, int64_t row, int64_t jb, int64_t je) {
+template <unsigned ORDER, bool WIDE, bool NARROW, bool FAST>
+__device__ __forceinline__ bool walk_directions(uint8_t *dir, const float *dem,
+                                                const float *dist, const int32_t *flats,
+                                                int64_t m, int64_t n, int64_t row, int64_t jb,
+                                                int cols, int lanes, int sl) {
   constexpr int R = kFlatR;
-  const int lane = threadIdx.x & 31;
   const bool rows_ok = row >= 0 && row < m;  // WIDE: m is a multiple of 4, all rows or none
-  const bool puts = rows_ok && lane >= 1 && lane < 31;
+  const bool puts = rows_ok && sl >= 1 && sl < lanes - 1;
+  const int64_t je = min(n, jb + cols);
+  const int64_t end = NARROW ? jb + cols : je;  // the strips of a warp walk in step
 
   bool odd = false;
   float nz[R], nd[R];  // the next column
@@ -363,7 +372,7 @@ __device__ __forceinline__ bool walk_directions(uint8_t *dir,
   // exactly as the reference skips them, so no bounds checks are needed.
   float z[3][R + 2] = {}, d[3][R + 2] = {};
   unsigned f[3] = {};
-  for (int64_t j0 = jb - 1; j0 < je + 1; j0 += 3) {
+  for (int64_t j0 = jb - 1; j0 < end + 1; j0 += 3) {
 #pragma unroll
     for (int b = 0; b < 3; b++) {
       const int64_t j = j0 + b;  // this column enters the window at index b
@@ -372,15 +381,15 @@ __device__ __forceinline__ bool walk_directions(uint8_t *dir,
       f[b] = 0;
 #pragma unroll
       for (int r = 0; r < R; r++) f[b] |= (unsigned)(nf[r] & 1) << r;
-      if (j < je) {
+      if (j < end) {
         flat_load<WIDE>(nz, dem, row, j + 1, m, n, rows_ok);
         flat_load<WIDE>(nd, dist, row, j + 1, m, n, rows_ok);
         flag_load<WIDE>(nf, flats, row, j + 1, m, n, rows_ok);
       }
-      z[b][0] = __shfl_up_sync(0xffffffffu, z[b][R], 1);
-      d[b][0] = __shfl_up_sync(0xffffffffu, d[b][R], 1);
-      z[b][R + 1] = __shfl_down_sync(0xffffffffu, z[b][1], 1);
-      d[b][R + 1] = __shfl_down_sync(0xffffffffu, d[b][1], 1);
+      z[b][0] = __shfl_up_sync(0xffffffffu, z[b][R], 1, lanes);
+      d[b][0] = __shfl_up_sync(0xffffffffu, d[b][R], 1, lanes);
+      z[b][R + 1] = __shfl_down_sync(0xffffffffu, z[b][1], 1, lanes);
+      d[b][R + 1] = __shfl_down_sync(0xffffffffu, d[b][1], 1, lanes);
       if (j - 1 >= jb && j - 1 < je) {  // directions of column j - 1
         const unsigned fm = f[(b + 2) % 3];
         const uint32_t o = column_directions<ORDER, FAST>(z, d, (b + 1) % 3, fm, odd);
@@ -400,20 +409,25 @@ __device__ __forceinline__ bool walk_directions(uint8_t *dir,
   return odd;
 }
 
-template <unsigned ORDER, bool WIDE>
+template <unsigned ORDER, bool WIDE, bool NARROW>
 __global__ void __launch_bounds__(kFlatWarps * 32)
 directions_kernel(uint8_t *dir, const float *dem,
                   const float *dist, const int32_t *flats, int64_t m,
-                  int64_t n, int strips, int cols) {
+                  int64_t n, int strips, int cols, int seg) {
   start_after_previous();
+  const int lane = threadIdx.x & 31;
   const int64_t w = (int64_t)blockIdx.x * kFlatWarps + (threadIdx.x >> 5);
-  const int64_t jb = w / strips * cols;  // first column put out
-  if (jb >= n) return;
-  const int64_t row = w % strips * kFlatRows + (int64_t)((int)(threadIdx.x & 31) - 1) * kFlatR;
-  const int64_t je = min(n, jb + cols);
-  const bool odd = walk_directions<ORDER, WIDE, true>(dir, dem, dist, flats, m, n, row, jb, je);
+  const int lanes = NARROW ? seg : 32, sl = NARROW ? lane & (seg - 1) : lane;
+  const int64_t first = NARROW ? w * (32 / seg) : w;
+  const int64_t walk = NARROW ? first + lane / seg : w;
+  const int64_t jb = walk / strips * cols;  // first column put out
+  if ((NARROW ? first / strips * cols : jb) >= n) return;
+  const int64_t row = walk % strips * ((lanes - 2) * kFlatR) + (int64_t)(sl - 1) * kFlatR;
+  const bool odd = walk_directions<ORDER, WIDE, NARROW, true>(dir, dem, dist, flats, m, n, row,
+                                                              jb, cols, lanes, sl);
   if (__any_sync(0xffffffffu, odd))  // rare: the same walk with divisions
-    walk_directions<ORDER, WIDE, false>(dir, dem, dist, flats, m, n, row, jb, je);
+    walk_directions<ORDER, WIDE, NARROW, false>(dir, dem, dist, flats, m, n, row, jb, cols, lanes,
+                                                sl);
 }
 
 // ------------------------------------------------------------------
@@ -791,16 +805,33 @@ hillshade_bwd_kernel(float *__restrict__ gdem, const float *__restrict__ dem,
 // and 48 within 5 %; 8 columns at least cost 512^2 0.2 us, 2 cost 0.5).
 // Directions, more work a column: 36 warps (4096^2 66 us, 70 with 24) and 2
 // columns (512^2 4.1 us, 4.4 with 4 and 5.7 with 8).
+//
+// A strip takes all 32 lanes of a warp and 120 rows, unless strips of 16, 8 or 4
+// lanes (56, 24 or 8 rows) leave at least a quarter fewer lanes without rows of
+// their own, as on grids of few rows or of a few rows more than whole strips:
+// 1 x 2^20 pixels flats 272 -> 41 us and directions 413 -> 61, 30 x 131072
+// 41 -> 25 and 62 -> 39, 127 x 40000 30 -> 25 and 46 -> 39.
 struct StripSplit {
-  int strips, cols;
+  int strips, cols, lanes;
   unsigned blocks;
 };
 StripSplit strip_split(const GridDims &g, int warps_per_sm, int least) {
-  StripSplit s{(int)((g.m + kFlatRows - 1) / kFlatRows), 64, 0};
+  auto strips_of = [&](int lanes) {
+    const int rows = (lanes - 2) * kFlatR;
+    return (int)((g.m + rows - 1) / rows);
+  };
+  int lanes = 32;
+  for (int l = 16; l >= 4; l /= 2) {
+    const int64_t now = (int64_t)strips_of(lanes) * lanes, then = (int64_t)strips_of(l) * l;
+    if (4 * then <= 3 * now) lanes = l;
+  }
+  StripSplit s{strips_of(lanes), 64, lanes, 0};
+  auto warps = [&] {
+    return (s.strips * ((g.n + s.cols - 1) / s.cols) + 32 / lanes - 1) / (32 / lanes);
+  };
   const int64_t want = (int64_t)sm_count() * warps_per_sm;
-  while (s.cols > least && s.strips * ((g.n + s.cols - 1) / s.cols) < want) s.cols /= 2;
-  const int64_t warps = s.strips * ((g.n + s.cols - 1) / s.cols);
-  s.blocks = (unsigned)((warps + kFlatWarps - 1) / kFlatWarps);
+  while (s.cols > least && warps() < want) s.cols /= 2;
+  s.blocks = (unsigned)((warps() + kFlatWarps - 1) / kFlatWarps);
   return s;
 }
 
@@ -821,13 +852,12 @@ tt_cuda_status identifyflats_dev(int32_t *flags, const float *dem,
   }
   // Wide accesses where every column of both arrays starts on a 16-byte boundary.
   const bool wide = g.m % 4 == 0 && (((uintptr_t)flags | (uintptr_t)dem) & 15) == 0;
-  const auto [strips, cols, blocks] = strip_split(g, 24, 4);
-  if (wide)
-    TT_LAUNCH_NEXT(identifyflats_kernel<true>, blocks, kFlatWarps * 32, 0, st, flags, dem, g.m, g.n,
-              strips, cols, slots);
-  else
-    TT_LAUNCH_NEXT(identifyflats_kernel<false>, blocks, kFlatWarps * 32, 0, st, flags, dem, g.m, g.n,
-              strips, cols, slots);
+  const StripSplit sp = strip_split(g, 24, 4);
+  const auto kernel =
+      sp.lanes < 32 ? (wide ? identifyflats_kernel<true, true> : identifyflats_kernel<false, true>)
+                    : (wide ? identifyflats_kernel<true, false> : identifyflats_kernel<false, false>);
+  TT_LAUNCH_NEXT(kernel, sp.blocks, kFlatWarps * 32, 0, st, flags, dem, g.m, g.n, sp.strips,
+                 sp.cols, sp.lanes, slots);
   if (count_dev) TT_LAUNCH(sum_slots_kernel, 1, 32, 0, st, slots, count_dev);
   TT_CHECK(cudaGetLastError());
   return TT_CUDA_SUCCESS;
@@ -839,11 +869,17 @@ tt_cuda_status directions_dev(uint8_t *dir, const float *dem, const float *dist,
   const bool wide =
       g.m % 4 == 0 && (((uintptr_t)dem | (uintptr_t)dist | (uintptr_t)flats) & 15) == 0 &&
       ((uintptr_t)dir & 3) == 0;
-  const auto [strips, cols, blocks] = strip_split(g, 36, 2);
-  const auto kernel = order & 1 ? (wide ? directions_kernel<1, true> : directions_kernel<1, false>)
-                                : (wide ? directions_kernel<0, true> : directions_kernel<0, false>);
-  TT_LAUNCH_NEXT(kernel, blocks, kFlatWarps * 32, 0, st, dir, dem, dist, flats, g.m, g.n, strips,
-            cols);
+  const StripSplit sp = strip_split(g, 36, 2);
+  auto pick = [&](auto ord) {
+    constexpr unsigned O = decltype(ord)::value;
+    return sp.lanes < 32
+               ? (wide ? directions_kernel<O, true, true> : directions_kernel<O, false, true>)
+               : (wide ? directions_kernel<O, true, false> : directions_kernel<O, false, false>);
+  };
+  const auto kernel = order & 1 ? pick(std::integral_constant<unsigned, 1>{})
+                                : pick(std::integral_constant<unsigned, 0>{});
+  TT_LAUNCH_NEXT(kernel, sp.blocks, kFlatWarps * 32, 0, st, dir, dem, dist, flats, g.m, g.n,
+                 sp.strips, sp.cols, sp.lanes);
   TT_CHECK(cudaGetLastError());
   return TT_CUDA_SUCCESS;
 }
