@@ -424,9 +424,10 @@ TT_CUDA_API tt_cuda_status tt_cuda_write_file_dev(const char *path, int64_t offs
  *  while they run -- a framework whose own memory pool already owns the
  *  device, or a loop that must not pay for cudaMalloc/cudaFree, which can
  *  synchronise the whole device.  The fill's scratch (a control block and
- *  one word per 32 x 32 tile, rounded up for each warp) lives in a static device array sized for
- *  65536 tiles (for example 8192 x 8192 pixels); each device that loads the
- *  library keeps it until the process exits.  Larger grids are rejected with
+ *  two words per 32 x 32 tile, rounded up for each warp) lives in a static
+ *  device array of 1 MiB, enough for 65536 tiles (for example 8192 x 8192
+ *  pixels); each device that loads the library keeps it until the process
+ *  exits.  Larger grids are rejected with
  *  TT_CUDA_ERR_INVALID_ARGUMENT.  The first call on a device looks up the
  *  array's device address (cudaGetSymbolAddress) with that device current;
  *  make that first call before any stream capture.  All calls share the

@@ -88,12 +88,8 @@ struct UpArgs {
   const uint8_t *dir;
   int64_t m, n;
   int tm, tn;
-  unsigned order;
   const float *w;  // nullptr: unit weights
   int wshift;      // fixed-point scale 2^wshift
-  int phase;       // 1: local pass (forest_up_kernel), 3: final pass (forest_fin_kernel)
-  bool want_acc;
-  bool want_h;
   CoarseCell *ccell;  // per exit id: sums, longest path, pending coarse donors
   CoarseCell *cell;   // per exit pixel: final totals, read by the final pass
   void *lacc;        // per pixel: in-tile (local) total, long long (int for unit counts)
@@ -160,10 +156,15 @@ __device__ __forceinline__ long long to_fixed(float w, int k, int *err) {
 //     its receivers to the in-tile terminal and records it with the number
 //     of steps (first pass only).
 constexpr int kUpThreads = 128;
-// Resident blocks per SM for the two tile passes (up to 56 and 40
-// registers a thread, no spills; shared memory allows 10 and 15): walks
-// wait at block barriers for the block's longest chain, so more resident
-// blocks keep the SM busy meanwhile.
+// Resident blocks per SM for the two tile passes: walks wait at block barriers
+// for the block's longest chain, so more resident blocks keep the SM busy
+// meanwhile, which is worth the spills that their 56 and 40 registers a thread
+// cost (4 to 48 bytes; shared memory allows 10 and 15 blocks).  First pass,
+// 8192^2 unit / weighted, 4096^2 with heights unit / weighted: 857 / 1162, 236 /
+// 311 us with nine blocks, 888 / 1206, 246 / 330 with eight (no spills), 840 /
+// 1155, 239 / 318 with ten.  Final pass: 283 / 467, 105 / 173 us with eleven
+// (the weighted ones spill), 311 / 449, 107 / 180 with ten, 313 / 454, 105 / 178
+// with nine: the weighted sum without heights alone would take ten.
 constexpr int kUpBlocks = 9;
 constexpr int kFinBlocks = 11;
 constexpr int kRing = 4 * kTile - 4;  // 124 ring pixels
@@ -1231,12 +1232,8 @@ tt_cuda_status up_run(const uint8_t *dir, const float *weights, int wshift,
   a.n = g.n;
   a.tm = g.tm;
   a.tn = g.tn;
-  a.order = order;
   a.w = weights;
   a.wshift = wshift;
-  a.phase = 1;
-  a.want_acc = want_acc;
-  a.want_h = want_h;
   a.ccell = w.ccell;
   a.cell = w.cell;
   a.lacc = w.lacc;
@@ -1301,7 +1298,6 @@ tt_cuda_status up_run(const uint8_t *dir, const float *weights, int wshift,
             w.ccell, w.counters + 2, (int)std::min<int64_t>(g.cells(), INT_MAX));
   TT_LAUNCH_NEXT(coarse_scatter_kernel, lg, 256, 0, st, w.counters + 0, w.elist, w.ccell,
             w.cell);
-  a.phase = 3;
   TT_LAUNCH_NEXT(fin, fgrid, kUpThreads, 0, st, a);
   TT_CHECK(cudaGetLastError());
   return TT_CUDA_SUCCESS;

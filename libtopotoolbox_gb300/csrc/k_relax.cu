@@ -584,12 +584,13 @@ relax_persistent_kernel(RelaxArgs a) {
         if (lane == l) atomicSub(&words[k], got);  // the lane that read this word
       }
     }
+    // ordered: the waiting tiles at or below the threshold
     for (int base = 0; ordered_sched(SCHED) && base < own && taken < kTakeTiles; base += 32) {
       const int mine = wid + (base + lane) * W;
       int f = f0;
       if (base) f = base + lane < own ? *(volatile int *)&words[base + lane] : 0;
       bool elig = f != 0;
-      if (ordered_sched(SCHED) && elig) {
+      if (elig) {
         const int pr = *(volatile int *)&a.prio[mine];
         elig = pr <= thr;
         // a flag whose priority was cleared by a take racing its publication
@@ -612,9 +613,9 @@ relax_persistent_kernel(RelaxArgs a) {
           fence_acq_rel_gpu();
         }
         const int got = __shfl_sync(0xffffffffu, f, l);
-        // ordered: clear the priority first, so a value published during the
-        // visit keeps one (at worst a stale one)
-        if (ordered_sched(SCHED) && lane == 0) atomicExch(&a.prio[tile], kClean);
+        // clear the priority first, so a value published during the visit
+        // keeps one (at worst a stale one)
+        if (lane == 0) atomicExch(&a.prio[tile], kClean);
         unflushed++;
         taken++;
         const bool fenced = relax_tile<KIND, SCHED>(a, t, lane, tile, got);
@@ -1215,11 +1216,15 @@ inline bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 inline bool aligned4(const void *p) { return ((uintptr_t)p & 3u) == 0; }
 
 // Smallest grid side that starts the fill from a coarse bound (0: never);
-// TT_CUDA_FILL_BOUND_MIN overrides it.  Measured on the 16384² workload
-// generator, without and with the bound: 16384² 7.16 and 6.39 ms, 12288² 4.20
-// and 3.99, 10240² 3.27 and 3.03, 8192² 2.19 and 2.17, 4096² 0.60 and 0.85
-// (the coarse run and the full first visit of every tile cost more than the
-// visits saved).
+// TT_CUDA_FILL_BOUND_MIN overrides it.  The coarse run and the full first visit
+// of every tile have to cost less than the visits they save, which depends on
+// the terrain; 12288 is the smallest side measured from which every terrain
+// gains.  ms without and with the bound on noise / metre steps / nodata / smooth
+// terrain: 8192^2 3.20 3.52 / 2.75 2.89 / 2.04 1.89 / 3.20 3.55, 9216^2 3.89
+// 3.16 / 3.49 2.79 / 2.69 2.52 / 3.78 3.12, 10240^2 4.17 3.90 / 3.67 4.02 /
+// 3.21 2.88 / 4.19 3.72, 12288^2 5.85 5.03 / 5.08 4.00 / 4.28 3.79 / 5.73 4.78.
+// Both sides count, so a long grid goes without, although 20000 x 10000 would
+// gain as well: 7.50 6.56 / 6.04 4.98 / 6.05 5.08 / 7.10 6.06.
 int64_t fill_bound_min() {
   static const int64_t v = [] {
     const char *s = std::getenv("TT_CUDA_FILL_BOUND_MIN");
@@ -1452,14 +1457,15 @@ tt_cuda_status gwdt_dev(float *dist, ptrdiff_t *prev, const float *costs,
 // For callers that cannot allocate device memory once they are running: a
 // framework whose own pool already holds the device's memory, or a loop
 // that must not pay for cudaMalloc/cudaFree (both can synchronise the whole
-// device).  The only scratch of the fill -- the control block and one word
-// per 32 x 32 tile, rounded up for each warp -- lives in the file-scope array
-// below, sized for kNoAllocMaxTiles tiles; every device that loads this library holds it
-// until the process exits.  All calls share it: each call clears what must
-// start at zero, and calls that overlap on the GPU race on it.  The array's
-// device address is looked up once per device and kept; a caller that
-// resets the device (cudaDeviceReset, which unloads this module) must not
-// call this entry point afterwards in the same process.
+// device).  The only scratch of the fill -- the control block and two words
+// per 32 x 32 tile (changes not taken in yet, and the lowest of them), rounded
+// up for each warp -- lives in the file-scope array below, sized for
+// kNoAllocMaxTiles tiles: 1 MiB that every device which loads this library
+// holds until the process exits.  All calls share it: each call clears what
+// must start at zero, and calls that overlap on the GPU race on it.  The
+// array's device address is looked up once per device and kept; a caller that
+// resets the device (cudaDeviceReset, which unloads this module) must not call
+// this entry point afterwards in the same process.
 // ------------------------------------------------------------------
 constexpr int kNoAllocMaxTiles = 65536;  // e.g. 8192 x 8192 pixels
 constexpr int kNoAllocMaxWarps = 8192;   // whose words are rounded up to whole sectors

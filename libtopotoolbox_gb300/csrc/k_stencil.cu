@@ -38,9 +38,10 @@ constexpr int kBlockY = 8;   // along j
 // from the lane's own rows and one shuffle each way, the flat bits of the rows
 // beside them from two ballots.  Nothing is staged in shared memory, and a
 // pixel costs some 20 operations instead of the 150 of a tile staged with its
-// halo and eight compares a pixel, which the ALU pipe bounded (85 % busy):
-// 16384^2 1.30 -> 0.45 ms (4.8 TB/s of 2.1 GB), 4096^2 84 -> 37 us, 3001 x 5003
-// 75 -> 42 us, 512^2 3.1 -> 3.6 us.
+// halo, which the ALU pipe bounded (85 % busy): 16384^2 1.51 ms with eight
+// compares a pixel there, 1.30 with shared minima, 0.45 so (4.8 TB/s of 2.1
+// GB); 4096^2 84 -> 37 us, 3001 x 5003 75 -> 42 us, 512^2 3.1 -> 3.6 us (both
+// after the 1.30).
 //
 // WIDE: 16-byte loads and stores, where every column starts on a 16-byte
 // boundary.  Elsewhere four strided ones, which L1 and L2 put together (one
