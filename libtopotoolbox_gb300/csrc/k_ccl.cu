@@ -51,19 +51,26 @@ __device__ __forceinline__ int uf_find(int *L, int x) {
   return x;
 }
 
+// Unites the components of a and b.  The greater label, where it is a root,
+// goes under the other one wherever that stands in its tree, so a row of tiles
+// that lie in one flat is linked up without a walk (the borders of a row or
+// column of 2^20 pixels 4 us; 1.6 to 2.1 ms when each union looked for both
+// roots first, up a chain of thousands of tiles); only where the greater one has
+// been linked before are the roots looked for.
 __device__ void uf_union(int *L, int a, int b) {
-  for (int it = 0; it < (1 << 30); it++) {
-    a = uf_find(L, a);
-    b = uf_find(L, b);
-    if (a == b) return;
-    if (a < b) {
-      int old = atomicMin(&L[b], a);
-      if (old == b) return;
-      b = old;
-    } else {
-      int old = atomicMin(&L[a], b);
-      if (old == a) return;
+  volatile int *vL = L;
+  a = vL[a];
+  b = vL[b];
+  for (int it = 0; it < (1 << 30) && a != b; it++) {
+    const int hi = max(a, b), lo = min(a, b);
+    if (vL[hi] == hi) {
+      const int old = atomicMin(&L[hi], lo);
+      if (old == hi) return;
       a = old;
+      b = lo;
+    } else {
+      a = uf_find(L, a);
+      b = uf_find(L, b);
     }
   }
 }
@@ -87,18 +94,19 @@ __device__ __forceinline__ int sfind(int *lab, int x) {
 }
 
 __device__ void sunion(int *lab, int a, int b) {
-  for (int it = 0; it < 4096; it++) {
-    a = sfind(lab, a);
-    b = sfind(lab, b);
-    if (a == b) return;
-    if (a < b) {
-      const int old = atomicMin(&lab[b], a);
-      if (old == b) return;
-      b = old;
-    } else {
-      const int old = atomicMin(&lab[a], b);
-      if (old == a) return;
+  volatile int *v = lab;
+  a = v[a];
+  b = v[b];
+  for (int it = 0; it < 4096 && a != b; it++) {
+    const int hi = max(a, b), lo = min(a, b);
+    if (v[hi] == hi) {
+      const int old = atomicMin(&lab[hi], lo);
+      if (old == hi) return;
       a = old;
+      b = lo;
+    } else {
+      a = sfind(lab, a);
+      b = sfind(lab, b);
     }
   }
 }
@@ -139,6 +147,14 @@ struct CclTile {
 struct __align__(16) LocalRoot {
   int pixel, key, arg, pad;
 };
+
+// The component of root pixel gp in the tile at (i0, j0), v its pack_best.
+__device__ __forceinline__ LocalRoot local_root(int gp, unsigned long long v, int64_t i0,
+                                                int64_t j0, int64_t m) {
+  const int a = 1023 - (int)(v & 1023u);
+  return LocalRoot{gp, v ? (int)((unsigned)(v >> 32) ^ 0x80000000u) : INT_MIN,
+                   v ? (int)((j0 + a / kTile) * m + (i0 + a % kTile)) : INT_MAX, 0};
+}
 
 __device__ __forceinline__ uint32_t run_starts(uint32_t m) { return m & ~(m << 1); }
 // First row of the run in slot k of a column with run starts s, -1 without one.
@@ -212,6 +228,35 @@ ccl_tile_kernel(int *__restrict__ L, unsigned long long *__restrict__ best,
     if (lane == 0) edges[tile] = make_uint4(top, bottom, t.mask[0], t.mask[kTile - 1]);
   }
   if (!some) return;  // no labels: L is only ever read at flat pixels
+
+  // A tile inside a flat is one component, of runs as long as they get, each of
+  // which one thread would scan: 4096^2 pixels of one flat 226 -> 55 us, a row
+  // of 2^20 262 -> 84 us, 16384^2 of metre steps 3.37 -> 2.88 ms.
+  const uint32_t all_rows = m - i0 >= kTile ? 0xffffffffu : (1u << (m - i0)) - 1u;
+  if (__all_sync(0xffffffffu, j0 + lane >= n || t.mask[lane] == all_rows)) {
+    const int first = (int)(j0 * m + i0);  // the root
+    int km = INT_MIN, kl = 0;
+#pragma unroll
+    for (int u = 0; u < kCols; u++) {
+      const int jj = warp * kCols + u, k = t.key[jj * kTile + lane];
+      if (i < m && j0 + jj < n) L[(j0 + jj) * m + i] = first;
+      if (k > km) {
+        km = k;
+        kl = jj * kTile + lane;
+      }
+    }
+    const int most = __reduce_max_sync(0xffffffffu, km);
+    const int at = __reduce_min_sync(0xffffffffu, km == most ? kl : INT_MAX);
+    if (lane == 0) t.best[warp] = most == INT_MIN ? 0ULL : pack_best(most, at);
+    __syncthreads();
+    if (tid == 0) {
+      unsigned long long v = t.best[0];
+      for (int w = 1; w < kCclThreads / 32; w++) v = max(v, t.best[w]);
+      roots[atomicAdd(nroots, 1)] = local_root(first, v, i0, j0, m);
+      best[first] = 0ULL;
+    }
+    return;
+  }
 
 #pragma unroll
   for (int q = 0; q < kSlotsPer; q++) {  // unions with the column before
@@ -289,10 +334,7 @@ ccl_tile_kernel(int *__restrict__ L, unsigned long long *__restrict__ best,
     const int slot = tid + q * kCclThreads, c = slot >> 4;
     if (root[q] != slot) continue;
     const int gp = (int)((j0 + c) * m + i0 + slot_row(run_starts(t.mask[c]), slot & 15));
-    const unsigned long long v = t.best[slot];
-    const int a = 1023 - (int)(v & 1023u);
-    roots[at++] = LocalRoot{gp, v ? (int)((unsigned)(v >> 32) ^ 0x80000000u) : INT_MIN,
-                            v ? (int)((j0 + a / kTile) * m + (i0 + a % kTile)) : INT_MAX, 0};
+    roots[at++] = local_root(gp, t.best[slot], i0, j0, m);
     best[gp] = 0ULL;
   }
 #pragma unroll
@@ -318,14 +360,25 @@ ccl_tile_kernel(int *__restrict__ L, unsigned long long *__restrict__ best,
 // their left column), and the two corners: (31, 31) against (0, 0) of the
 // tile below-right, (31, 0) against (0, 31) of the tile below-left.
 //
-// One warp per tile, a lane per run of each border.  A union is a chain of
-// dependent accesses, so the pass takes as long as the most unions in one
-// thread: a thread per tile, with up to 32 of them, took 51 us at 512^2 and
-// 78 us at 3001 x 5003, a lane per run takes 10 and 21 us.
+// A warp takes `per` tiles and a lane a run at a time of all their borders.  A
+// union is a chain of dependent accesses, so on small grids the pass takes as
+// long as the most unions in one thread (512^2 9 us with a tile a warp, 17 with
+// four, 65 with 32), and on large ones, where most tiles have few runs or none,
+// as long as the warps that find few: 16384^2 of metre steps 358, 264, 225, 250
+// and 317 us with 1, 2, 4, 8 and 32 tiles a warp, of noise 219, 148, 103, 88 and
+// 117.  So a tile a warp until the SMs hold 48 warps each, then up to four.
+constexpr int kBorderWarps = 8;
+constexpr int kBorderTiles = 4;           // most tiles a warp
+constexpr int kBorderItems = 2 * 16 + 2;  // runs of two borders and two corners
+
+struct BorderWarp {
+  uint4 mask[kBorderTiles];  // bottom row, top row below, right column, left column beside
+  uint16_t item[kBorderTiles * kBorderItems];  // tile << 7 | kind << 5 | first bit
+};
+
 __device__ __forceinline__ void unite_run(int *L, uint32_t a, uint32_t b, int s0, int64_t pa0,
                                           int64_t pa_step, int64_t pb0, int64_t pb_step) {
-  if (!((a & ~(a << 1)) >> s0 & 1u)) return;  // no run of a starts here
-  const uint32_t sb = b & ~(b << 1);          // run starts of b
+  const uint32_t sb = b & ~(b << 1);  // run starts of b
   const uint32_t rm = run_mask(a, s0);
   uint32_t ov = b & (rm | (rm << 1) | (rm >> 1));
   while (ov) {
@@ -335,30 +388,67 @@ __device__ __forceinline__ void unite_run(int *L, uint32_t a, uint32_t b, int s0
   }
 }
 
-__global__ void ccl_border_kernel(int *L, const uint4 *edges,
-                                  int64_t m, int tm, int tn) {
+__global__ void __launch_bounds__(kBorderWarps * 32)
+ccl_border_kernel(int *L, const uint4 *edges, int64_t m, int tm, int tn, int per) {
+  __shared__ BorderWarp warps[kBorderWarps];
   start_after_previous();
+  BorderWarp &w = warps[threadIdx.x >> 5];
   const int T = tm * tn;
   const int lane = threadIdx.x & 31;
-  const int tile = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-  if (tile >= T) return;
-  const int ti = tile % tm, tj = tile / tm;
-  const int64_t i0 = (int64_t)ti * kTile, j0 = (int64_t)tj * kTile;
-  // the three tiles' masks in one round trip
-  const uint32_t d = ti + 1 < tm ? edges[tile + 1].x : 0u;   // the tile below
-  const uint32_t r = tj + 1 < tn ? edges[tile + tm].z : 0u;  // the tile to the right
-  const uint4 e = edges[tile];                               // top, bottom, left, right
-  if (ti + 1 < tm && e.y) {
-    if (d)  // bottom row (i0 + 31, j0 + k) against row i0 + 32
-      unite_run(L, e.y, d, lane, j0 * m + i0 + kTile - 1, m, j0 * m + i0 + kTile, m);
-    if (lane == 0 && tj + 1 < tn && (e.y >> 31) && (edges[tile + 1 + tm].x & 1u))
-      uf_union(L, (int)((j0 + kTile - 1) * m + i0 + kTile - 1),
-               (int)((j0 + kTile) * m + i0 + kTile));
-    if (lane == 1 && tj > 0 && (e.y & 1u) && (edges[tile + 1 - tm].x >> 31))
-      uf_union(L, (int)(j0 * m + i0 + kTile - 1), (int)((j0 - 1) * m + i0 + kTile));
+  const int64_t first = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * per;
+  if (first >= T) return;
+  uint4 e = {};                              // top, bottom, left, right of this lane's tile
+  uint32_t d = 0, r = 0, below = 0, above = 0;
+  if (lane < per && first + lane < T) {
+    const int tile = (int)first + lane, ti = tile % tm, tj = tile / tm;
+    // the five tiles' masks in one round trip
+    e = edges[tile];
+    if (ti + 1 < tm) {
+      d = edges[tile + 1].x;
+      if (tj + 1 < tn) below = edges[tile + 1 + tm].x & 1u;
+      if (tj > 0) above = edges[tile + 1 - tm].x >> 31;
+    }
+    if (tj + 1 < tn) r = edges[tile + tm].z;
   }
-  if (e.w && r)  // right column (i0 + k, j0 + 31) against column j0 + 32
-    unite_run(L, e.w, r, lane, (j0 + kTile - 1) * m + i0, 1, (j0 + kTile) * m + i0, 1);
+  if (lane < per) w.mask[lane] = make_uint4(e.y, d, e.w, r);
+  const uint32_t down = d ? run_starts(e.y) : 0u, right = r ? run_starts(e.w) : 0u;
+  below &= e.y >> 31;
+  above &= e.y & 1u;
+  const int mine = __popc(down) + __popc(right) + (int)below + (int)above;
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  int at = incl - mine;
+  for (uint32_t s = down; s; s &= s - 1) w.item[at++] = (uint16_t)(lane << 7 | (__ffs(s) - 1));
+  for (uint32_t s = right; s; s &= s - 1)
+    w.item[at++] = (uint16_t)(lane << 7 | 1 << 5 | (__ffs(s) - 1));
+  if (below) w.item[at++] = (uint16_t)(lane << 7 | 2 << 5);
+  if (above) w.item[at++] = (uint16_t)(lane << 7 | 3 << 5);
+  __syncwarp();
+  for (int k = lane; k < total; k += 32) {
+    const int item = w.item[k], s0 = item & 31;
+    const int tile = (int)first + (item >> 7), ti = tile % tm, tj = tile / tm;
+    const int64_t i0 = (int64_t)ti * kTile, j0 = (int64_t)tj * kTile;
+    const uint4 b = w.mask[item >> 7];
+    switch ((item >> 5) & 3) {
+      case 0:  // bottom row (i0 + 31, j0 + k) against row i0 + 32
+        unite_run(L, b.x, b.y, s0, j0 * m + i0 + kTile - 1, m, j0 * m + i0 + kTile, m);
+        break;
+      case 1:  // right column (i0 + k, j0 + 31) against column j0 + 32
+        unite_run(L, b.z, b.w, s0, (j0 + kTile - 1) * m + i0, 1, (j0 + kTile) * m + i0, 1);
+        break;
+      case 2:
+        uf_union(L, (int)((j0 + kTile - 1) * m + i0 + kTile - 1),
+                 (int)((j0 + kTile) * m + i0 + kTile));
+        break;
+      default:
+        uf_union(L, (int)(j0 * m + i0 + kTile - 1), (int)((j0 - 1) * m + i0 + kTile));
+    }
+  }
 }
 
 // A component's maximum depth key and the smallest pixel attaining it,
@@ -498,7 +588,10 @@ tt_cuda_status costs_dev(float *costs, ptrdiff_t *conncomps,
   // takes longer (many runs, many unions)
   TT_LAUNCH(ccl_tile_kernel, T, kCclThreads, 0, st, L, best, roots, nroots, edges, flats, orig,
             filled, g.m, g.n, g.tm);
-  TT_LAUNCH_NEXT(ccl_border_kernel, (T + 7) / 8, 256, 0, st, L, edges, g.m, g.tm, g.tn);
+  const int per = std::max(1, std::min(kBorderTiles, T / (sm_count() * 48)));
+  const int bwarps = (T + per - 1) / per;
+  TT_LAUNCH_NEXT(ccl_border_kernel, (bwarps + kBorderWarps - 1) / kBorderWarps,
+                 kBorderWarps * 32, 0, st, L, edges, g.m, g.tm, g.tn, per);
   TT_LAUNCH_NEXT(ccl_root_kernel, grid, 256, 0, st, L, roots, nroots, best);
   const int cgrid = (int)std::min<int64_t>((N + 1023) / 1024, (int64_t)sm_count() * 32);
   if (seed)
