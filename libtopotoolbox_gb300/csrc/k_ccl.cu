@@ -485,16 +485,16 @@ __global__ void ccl_root_kernel(int *L, const LocalRoot *roots,
   }
 }
 
-// Two pixels per thread: each level of the dependent gather (a pixel's
-// local root, its global root, the root's maximum and argmax) is issued for
-// both before any result is used.  16384^2 takes 1.52 ms so, 1.65 with four
-// and 1.93 with one; 4096^2 112, 129 and 135 us.  Tiles instead of runs of
+// Several pixels per thread: each level of the dependent gather (a pixel's
+// local root, its global root, the root's maximum and argmax) is issued for all
+// before any result is used.  Two where the gwdt start is written: 16384^2
+// takes 1.52 ms so, 1.65 with four and 1.93 with one; 4096^2 112, 129 and 135
+// us.  Four for the costs and labels alone: 16384^2 1.41 ms, 1.53 with two (of
+// metre steps 1.51 and 1.58), 512^2 4.2 and 4.9 us.  Tiles instead of runs of
 // pixels (2.04 ms), 16-byte vectors of four (1.57) and roots that carry their
-// component's maximum, one level less (1.96 + 0.10), were slower.  Labels are read at flat pixels only
-// (the labelling writes none elsewhere); `conncomps` may be null (the
-// pipeline needs the costs alone).
-constexpr int kCostPer = 2;
-
+// component's maximum, one level less (1.96 + 0.10), were slower.  Labels are
+// read at flat pixels only (the labelling writes none elsewhere); `conncomps`
+// may be null (the pipeline needs the costs alone).
 template <bool SEED>
 __global__ void costs_kernel(float *costs,
                              ptrdiff_t *conncomps, int *L,
@@ -504,6 +504,7 @@ __global__ void costs_kernel(float *costs,
                              const float *filled, int64_t N,
                              GwdtSeed seed, int64_t m, int64_t n, int tm) {
   start_after_previous();
+  constexpr int kCostPer = SEED ? 2 : 4;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p0 < N;
        p0 += kCostPer * stride) {
