@@ -237,8 +237,9 @@ __global__ void sum_slots_kernel(const unsigned long long *__restrict__ slots,
 // floats further the exact quotients lie 1.4 units of the last place apart).
 // The direction is the first neighbour in order that reaches the largest
 // slope.  Quotients are a reciprocal product with an exact remainder; a warp
-// that meets a drop below 2^-100, where that remainder would underflow, takes
-// its columns again with divisions.
+// that meets a drop below 2^-100, where that remainder would underflow, stops
+// and takes its columns again with divisions (4096^2 of such drops 197 us, 232
+// when it went on to its last column first).
 //
 // Warps walk along strips of rows as in identifyflats_kernel, dem and dist of
 // three columns in registers and the next one loaded ahead (three ahead take
@@ -351,7 +352,8 @@ __device__ __forceinline__ uint32_t column_directions(const float (&z)[3][kFlatR
 }
 
 // Directions of columns jb .. jb + cols - 1 of the strip whose rows start at `row` in
-// this lane.  Returns whether a quotient of this lane may not hold.
+// this lane.  Returns whether a quotient may not hold (FAST: as soon as one of the
+// warp's does not).
 template <unsigned ORDER, bool WIDE, bool NARROW, bool FAST>
 __device__ __forceinline__ bool walk_directions(uint8_t *dir, const float *dem,
                                                 const float *dist, const int32_t *flats,
@@ -406,6 +408,7 @@ __device__ __forceinline__ bool walk_directions(uint8_t *dir, const float *dem,
         }
       }
     }
+    if (FAST && __any_sync(0xffffffffu, odd)) return true;  // walked again anyway
   }
   return odd;
 }
