@@ -260,10 +260,14 @@ template <class S>
 __device__ __forceinline__ typename S::T sum_needed(const FlowArgs &a, const EdgeRec &r) {
   typename S::T s = S::start(r.w);
   const unsigned long long *val = a.val + r.in_lo;
+  unsigned long long b[kReadAhead];
+  read_ahead(val, r.need, b);
   for (int k = 0; k < r.need; k += kReadAhead) {
-    unsigned long long b[kReadAhead];
-    read_ahead(val + k, r.need - k, b);
+    unsigned long long next[kReadAhead];  // on their way while these are added
+    read_ahead(val + k + kReadAhead, r.need - k - kReadAhead, next);
     s = add_ahead<S>(a, val + k, r.need - k, b, s);
+#pragma unroll
+    for (int u = 0; u < kReadAhead; u++) b[u] = next[u];
   }
   return s;
 }
