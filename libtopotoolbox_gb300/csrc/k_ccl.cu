@@ -170,9 +170,9 @@ __device__ __forceinline__ int slot_row(uint32_t s, int k) {
 // parts -- unions, and a run's best pixel -- are at most four runs a thread;
 // a warp per tile with a lane per column stepped through up to sixteen, half
 // of its lanes idle (14.7 of 32 active), and took 39 us for any grid, however
-// small.  (512^2 39 -> 17 us, 4096^2 191 -> 174 us, 16384^2 2.64 -> 2.31 ms;
-// ten blocks an SM: 2.45 ms with eight, 2.25 with fourteen, which is slower
-// on the smaller grids.)
+// small.  (512^2 39 -> 17 us, 4096^2 191 -> 174 us, 16384^2 2.64 -> 2.31 ms, and
+// 1.97 with the tiles inside a flat taken as a whole; ten blocks an SM: 2.45 ms
+// with eight, 2.25 with fourteen, which is slower on the smaller grids.)
 // Each tile-local component is reduced to its maximum depth and the smallest
 // pixel attaining it, and every flat pixel takes its component's root.
 __global__ void __launch_bounds__(kCclThreads, 10)
