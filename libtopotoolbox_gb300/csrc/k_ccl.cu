@@ -93,20 +93,22 @@ __device__ __forceinline__ int sfind(int *lab, int x) {
   return x;
 }
 
+// Roots first: a link at the raw label, as across tiles, deepens the trees, on
+// which a small grid's slowest tile waits (300^2 of noise 14.6 -> 16.8 us, 1024^2
+// of metre steps 20 -> 23; 4096^2 196 -> 184).
 __device__ void sunion(int *lab, int a, int b) {
-  volatile int *v = lab;
-  a = v[a];
-  b = v[b];
-  for (int it = 0; it < 4096 && a != b; it++) {
-    const int hi = max(a, b), lo = min(a, b);
-    if (v[hi] == hi) {
-      const int old = atomicMin(&lab[hi], lo);
-      if (old == hi) return;
-      a = old;
-      b = lo;
+  for (int it = 0; it < 4096; it++) {
+    a = sfind(lab, a);
+    b = sfind(lab, b);
+    if (a == b) return;
+    if (a < b) {
+      const int old = atomicMin(&lab[b], a);
+      if (old == b) return;
+      b = old;
     } else {
-      a = sfind(lab, a);
-      b = sfind(lab, b);
+      const int old = atomicMin(&lab[a], b);
+      if (old == a) return;
+      a = old;
     }
   }
 }
@@ -231,7 +233,7 @@ ccl_tile_kernel(int *__restrict__ L, unsigned long long *__restrict__ best,
 
   // A tile inside a flat is one component, of runs as long as they get, each of
   // which one thread would scan: 4096^2 pixels of one flat 226 -> 55 us, a row
-  // of 2^20 262 -> 84 us, 16384^2 of metre steps 3.37 -> 2.88 ms.
+  // of 2^20 262 -> 85 us, 16384^2 of metre steps 3.37 -> 2.86 ms.
   const uint32_t all_rows = m - i0 >= kTile ? 0xffffffffu : (1u << (m - i0)) - 1u;
   if (__all_sync(0xffffffffu, j0 + lane >= n || t.mask[lane] == all_rows)) {
     const int first = (int)(j0 * m + i0);  // the root
